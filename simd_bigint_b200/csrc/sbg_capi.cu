@@ -137,6 +137,23 @@ static int run_conv(sbg_ctx* c, uint64_t* rp, const uint64_t* ap, int64_t an, co
     if (lgL > SBG_NCODES || code_len(lgL) > ((int64_t)1 << SBG_MAX_LG)) return SBG_EBAND;
     int st = ensure_plan(c, lgL);
     if (st) return st;
+    if (lgL >= SBG_FUSED_MIN_LG && lgL <= SBG_SMALL_MAX_LG) {
+        if (b_ready) CK(cudaStreamWaitEvent(c->stream, b_ready, 0));
+        JobDesc J{};
+        J.a = ap;
+        J.b = bp;
+        J.out = rp;
+        J.an = an;
+        J.bn = bn;
+        J.cmin = cmin;
+        J.cmax = cmax;
+        J.off = off;
+        J.nout = nout;
+        J.sq = sq;
+        CK(launch_fused(J, lgL, &c->plans[lgL], c->tw_f, c->tw_i, c->err, c->stream, c->timer));
+        c->launches += 1;
+        return SBG_OK;
+    }
     st = ensure_ws(c, ws_words(lgL, sq), carry_flag_words(nout));
     if (st) return st;
     const LenPlan* lp = &c->plans[lgL];

@@ -1,0 +1,287 @@
+// sbg_fused.cuh -- a whole product of 2^8 <= L <= 2^12 transform points in
+// one launch (included by sbg_kernels.cu).
+//
+// A cluster of five CTAs, one per prime.  Each CTA transforms both operands,
+// multiplies and transforms back in shared memory (the operands side by side
+// on 256 threads each, radix-16 groups straight from the limbs, the last
+// forward pass, the product and the first inverse pass fused in registers;
+// twiddles staged in shared memory, since a single product touches each only
+// once or twice and would wait for each level's from L2).  The five CTAs
+// then read each other's residues through distributed shared memory, rebuild
+// the coefficients (two per thread) and resolve the carries: a warp's by
+// ballots, the cluster's from the (generate, propagate) bits of all its
+// warps.  Nothing goes through global memory between the limbs and the
+// product, and no flag is waited for.
+// What bounds it is the chain of passes on five SMs (20,000 clocks at 2^12
+// points, the SMs issuing 44% of them), so it is the single product's path;
+// batches fill the device with one CTA per prime and a separate carry scan.
+// 1500 x 1500 limbs, device time a call back to back: 30.7 us with the
+// transforms, the flags' memset and the carry scan as three launches, 12.3 us.
+// Shorter transforms (2^4 .. 2^7, tiny middle products) keep those launches.
+#pragma once
+
+namespace sbg {
+
+#define FU_T 512
+#define FU_V 2                                 // limbs per thread in the carry phase
+
+template <int LG>
+struct FusedSmem {
+    uint32_t A[padded_len(1 << LG)];
+    uint32_t B[padded_len(1 << LG)];
+    uint2 twf[1 << LG];
+    uint2 twi[1 << LG];
+    ulonglong2 xlo[FU_T / 32][2];              // limbs of each warp's last two lanes
+    uint64_t xmid[FU_T / 32][2];
+    uint2 xhi[FU_T / 32][2];
+    uint32_t warp[FU_T / 32];                  // (G, P) of this CTA's warps
+};
+
+__device__ __forceinline__ uint32_t dsmem_ld(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];\n" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+
+// one middle pass (both operands or the product) of a transform in shared memory
+template <int LG, int K, bool FWD>
+__device__ __forceinline__ void fused_pass(uint32_t* buf, int gid, SharedTw tw, uint32_t p) {
+    constexpr int r = prl(LG, K), R = 1 << r, LGM = lgm_of(LG, K), LGST = LGM - r, ST = 1 << LGST;
+    const int j0 = gid & (ST - 1), i0 = ((gid >> LGST) << LGM) + j0;
+    uint32_t x[R];
+#pragma unroll
+    for (int t = 0; t < R; ++t) x[t] = buf[padded_at<LGST>(i0, t)];
+    if constexpr (FWD)
+        dif_regs<R, ST == 1>(x, tw, j0, ST, LGM, p);
+    else
+        dit_regs<R, ST == 1>(x, tw, j0, ST, LGM, p);
+#pragma unroll
+    for (int t = 0; t < R; ++t) buf[padded_at<LGST>(i0, t)] = x[t];
+}
+
+template <int LG>
+__device__ __forceinline__ void fused_body(int q, const JobDesc& J, const uint2* __restrict__ twf,
+                                           const uint2* __restrict__ twi, uint32_t scw, uint32_t scws,
+                                           uint32_t* err) {
+    extern __shared__ __align__(16) uint8_t fu_raw[];
+    FusedSmem<LG>& S = *reinterpret_cast<FusedSmem<LG>*>(fu_raw);
+    constexpr int L = 1 << LG, NP = num_passes(LG), NG = L / 16;     // radix-16 groups per operand
+    static_assert(NP == 2 || NP == 3, "two or three passes");
+    constexpr unsigned FULL = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const PrimeConst pc = c_pr[q];
+    const uint32_t p = pc.p;
+
+    // twiddles of every size up to L: 16-byte asynchronous copies
+    for (int i = tid; i < L; i += FU_T) {
+        const int h = i >= L / 2;
+        const int e = 2 * (h ? i - L / 2 : i);
+        const uint2* src = (h ? twi : twf) + (size_t)q * SBG_TW_N + e;
+        const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared((h ? S.twi : S.twf) + e));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    const SharedTw sf{S.twf}, si{S.twi};
+    // the reconstruction's constants, fetched while the operands are
+    uint32_t touch = 0;
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(CrtConst) / 4; i += 16) touch |= reinterpret_cast<const uint32_t*>(&c_crt)[i];
+    asm volatile("" ::"r"(touch));
+    // first pass: limbs -> residues -> four levels
+    const int op = tid / NG, gid = tid & (NG - 1);
+    const bool in_op = op < (J.sq ? 1 : 2);
+    constexpr int ST0 = L / 16;
+    const int xn = (int)(op ? J.bn : J.an);
+    uint32_t x0[16];
+    if (in_op) {
+        const uint64_t* X = op ? J.b : J.a;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            const int n = gid + ST0 * t;
+            x0[t] = n < xn ? limb_residue(__ldcg(&X[n]), pc) : 0u;
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    if (in_op) {
+        if (xn <= L / 2)
+            dif_regs<16, false, true>(x0, sf, gid, ST0, LG, p);
+        else
+            dif_regs<16>(x0, sf, gid, ST0, LG, p);
+        uint32_t* buf = op ? S.B : S.A;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) buf[padded_at<LG - 4>(gid, t)] = x0[t];
+    }
+    __syncthreads();
+    if constexpr (NP == 3) {
+        if (in_op) fused_pass<LG, 1, true>(op ? S.B : S.A, gid, sf, p);
+        __syncthreads();
+    }
+    // last forward pass, product times the CRT scale, first inverse pass
+    {
+        constexpr int K = NP - 1, r = prl(LG, K), R = 1 << r;
+        for (int g = tid; g < L / R; g += FU_T) {
+            const int i0 = g << r;
+            uint32_t x[R], y[R];
+#pragma unroll
+            for (int t = 0; t < R; ++t) x[t] = S.A[padded_at<0>(i0, t)];
+            if (J.sq) {
+                dif_regs<R, true>(x, sf, 0, 1, r, p);
+#pragma unroll
+                for (int t = 0; t < R; ++t) y[t] = x[t];
+            } else {
+#pragma unroll
+                for (int t = 0; t < R; ++t) y[t] = S.B[padded_at<0>(i0, t)];
+                dif_regs2<R, true>(x, y, sf, 0, 1, r, p);
+            }
+#pragma unroll
+            for (int t = 0; t < R; ++t) x[t] = mul_shoup(mont_mul(x[t], y[t], p, pc.pinv), scw, scws, p);
+            dit_regs<R, true>(x, si, 0, 1, r, p);
+#pragma unroll
+            for (int t = 0; t < R; ++t) S.A[padded_at<0>(i0, t)] = x[t];
+        }
+    }
+    __syncthreads();
+    if constexpr (NP == 3) {
+        if (tid < NG) fused_pass<LG, 1, false>(S.A, tid, si, p);
+        __syncthreads();
+    }
+    if (tid < NG) fused_pass<LG, 0, false>(S.A, tid, si, p);
+    cluster_barrier<true>();                   // every prime's residues are in shared memory
+
+    // Coefficients -> limbs.  Limbs 0 .. nout (nout: the spill check) go to the
+    // five CTAs in equal runs; a CTA's threads take two consecutive limbs each
+    // from four below its run, whose coefficients the run's first limbs need.
+    const int nout = (int)J.nout, off = (int)J.off, cmin = (int)J.cmin, cmax = (int)J.cmax;
+    const int run = ((nout + SBG_NP) / SBG_NP + 1) & ~1;
+    const int c0 = q * run, c1 = min(c0 + run, nout + 1);
+    const int m0 = c0 - 4 + FU_V * tid;
+    const bool on = c0 - 4 + FU_V * 32 * wid < c1;         // warps beyond the run have nothing to do
+    const uint32_t inj = *(volatile uint32_t*)&g_inject;
+    uint64_t lo[FU_V] = {}, mid[FU_V] = {}, z[FU_V] = {};
+    uint32_t hi[FU_V] = {}, gb = 0, pb = 0, vbad = 0, wg = 0, wp = 0;
+    if (on) {
+        uint32_t r[FU_V][SBG_NP];
+#pragma unroll
+        for (int k = 0; k < SBG_NP; ++k) {
+            const uint32_t base = dsmem_addr(S.A, k);
+#pragma unroll
+            for (int i = 0; i < FU_V; ++i) {
+                const int j = m0 + i + off;
+                r[i][k] = m0 + i < c1 && j >= cmin && j <= cmax ? dsmem_ld(base + 4u * pad_idx(j)) : 0u;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < FU_V; ++i) {
+            const int j = m0 + i + off;
+            if (inj && j >= cmin && j <= cmax &&
+                (((inj & SBG_INJECT_TOP) && j == cmax) || ((inj & SBG_INJECT_MID) && j == cmin + (cmax - cmin) / 2)))
+                r[i][0] ^= 1u;
+            garner(r[i], lo[i], mid[i], hi[i]);
+        }
+        if (lane >= 30) {                      // what the warp above takes from this one
+            S.xlo[wid][lane - 30] = make_ulonglong2(lo[1], mid[0]);
+            S.xmid[wid][lane - 30] = mid[1];
+            S.xhi[wid][lane - 30] = make_uint2(hi[0], hi[1]);
+        }
+    }
+    __syncthreads();
+    if (on) {
+        uint64_t b_mid1 = __shfl_up_sync(FULL, mid[1], 1);
+        uint32_t b_hi0 = __shfl_up_sync(FULL, hi[0], 1), b_hi1 = __shfl_up_sync(FULL, hi[1], 1), c_k1 = 0;
+        if (lane == 0 && wid > 0) {
+            uint64_t t;
+            const ulonglong2 l = S.xlo[wid - 1][1];
+            const uint2 h = S.xhi[wid - 1][1];
+            b_mid1 = S.xmid[wid - 1][1];
+            b_hi0 = h.x;
+            b_hi1 = h.y;
+            sum3(l.x, l.y, S.xhi[wid - 1][0].y, t, c_k1);  // the sum carry of the limb below
+        }
+        if (lane == 0 && wid == 0) b_mid1 = b_hi0 = b_hi1 = 0;
+        uint64_t y[FU_V];
+        uint32_t kk[FU_V];
+        sum3(lo[0], b_mid1, b_hi0, y[0], kk[0]);
+        sum3(lo[1], mid[0], b_hi1, y[1], kk[1]);
+        uint32_t b_k1 = __shfl_up_sync(FULL, kk[1], 1);
+        if (lane == 0) b_k1 = c_k1;
+        if (m0 == 0) b_k1 = 0;                 // limb -1 carries nothing into limb 0
+#pragma unroll
+        for (int i = 0; i < FU_V; ++i) {
+            const int m = m0 + i;
+            z[i] = y[i] + (i == 0 ? b_k1 : kk[0]);
+            uint32_t G = z[i] < y[i], P = z[i] == ~0ull;
+            if (m >= nout) {
+                if (m == nout) vbad = G | kk[i];           // must end zero with no carry beyond it
+                G = 0;
+                P = 0;
+            }
+            if (m < c0 || m >= c1) {           // not of this run: passes the carry on
+                G = 0;
+                P = 1;
+            }
+            gb |= G << i;
+            pb |= P << i;
+        }
+        const uint32_t lG = (pb + (gb << 1)) >> FU_V, lP = pb == (1u << FU_V) - 1u;
+        wg = __ballot_sync(FULL, lG & 1u);
+        wp = __ballot_sync(FULL, lP);
+        if (lane == 0) {
+            const uint32_t G = (uint32_t)(((uint64_t)wp + (wg << 1)) >> 32) | (wg >> 31);
+            S.warp[wid] = (G & 1u) | ((wp == FULL) << 1);
+        }
+    } else if (lane == 0) {
+        S.warp[wid] = 2u;                      // identity
+    }
+    cluster_barrier<true>();                   // all warps' (G, P) are in shared memory
+    // the carry into this warp: over the CTAs below, then this CTA's warps
+    uint32_t v[SBG_NP], cin = 0, cw = 0;
+#pragma unroll
+    for (int k = 0; k < SBG_NP; ++k)
+        v[k] = k <= q && lane < FU_T / 32 ? dsmem_ld(dsmem_addr(S.warp, k) + 4 * lane) : 2u;
+#pragma unroll
+    for (int k = 0; k < SBG_NP; ++k) {
+        const uint32_t g = __ballot_sync(FULL, v[k] & 1u) & 0xffffu, pr = __ballot_sync(FULL, v[k] & 2u) & 0xffffu;
+        const uint32_t sum = pr + ((g << 1) | cin);
+        if (k == q) cw = (sum ^ pr) >> wid;
+        cin = ((sum >> (FU_T / 32)) | (g >> (FU_T / 32 - 1))) & 1u;
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");     // peers' memory is read
+    if (on) {
+        const uint32_t c = cw & 1u;
+        const uint64_t sum = (uint64_t)wp + ((wg << 1) | c);
+        const uint32_t cl = (((uint32_t)sum ^ wp) >> lane) & 1u;
+        const uint32_t cm = (pb + ((gb << 1) | cl)) ^ pb;
+#pragma unroll
+        for (int i = 0; i < FU_V; ++i) {
+            const int m = m0 + i;
+            const uint64_t w = z[i] + ((cm >> i) & 1u);
+            if (m < c0 || m >= c1) continue;
+            if (m < nout)
+                J.out[m] = w;
+            else if (vbad | (w != 0) | (w < z[i]))
+                atomicOr(err, 2u);
+        }
+    }
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");       // peers may still read ours
+}
+
+template <int LG>
+__global__ void __launch_bounds__(FU_T, 1) k_fused(const __grid_constant__ JobDesc J, const uint2* __restrict__ twf,
+                                                   const uint2* __restrict__ twi, ScaleArg sc, uint32_t* err) {
+    fused_body<LG>(blockIdx.x, J, twf, twi, sc.w[blockIdx.x], sc.ws[blockIdx.x], err);
+}
+
+#define SBG_FUSED_CASES(X) X(8) X(9) X(10) X(11) X(12)
+
+static cudaError_t fused_attr() {
+    cudaError_t e = cudaSuccess;
+#define SBG_FUSED_ATTR(n) \
+    if (e == cudaSuccess) \
+        e = cudaFuncSetAttribute(k_fused<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FusedSmem<n>));
+    SBG_FUSED_CASES(SBG_FUSED_ATTR)
+#undef SBG_FUSED_ATTR
+    return e;
+}
+
+}  // namespace sbg

@@ -220,6 +220,11 @@ cudaError_t launch_u52_decode(uint64_t* d, int64_t n52, const uint64_t* a, int64
 size_t u52_encode_scratch_words(int64_t rn);
 cudaError_t launch_u52_encode(uint64_t* r, int64_t rn, const uint64_t* d, int64_t n52, int sgn,
                               uint32_t* scratch, cudaStream_t st);
+// A whole product of SBG_FUSED_MIN_LG <= lgL <= SBG_SMALL_MAX_LG in one launch
+// (J.ws and J.flags are not used).
+#define SBG_FUSED_MIN_LG 8
+cudaError_t launch_fused(const JobDesc& J, int lgL, const LenPlan* lp, const uint2* tw_f, const uint2* tw_i,
+                         uint32_t* err, cudaStream_t st, KTimer* kt = nullptr);
 int64_t crt_blocks(int64_t nout);
 // All stages of one size class of the batch engine (every job of length
 // 2^lgL); `flags` holds flag_words zero-initialised words, job regions inside.

@@ -1641,6 +1641,10 @@ __global__ void __launch_bounds__(CRT_T, CRT_MINB) k_crt_carry_b(const JobDesc* 
     crt_body(s_bid, J.ws, L, J.cmin, J.cmax, J.off, J.out, J.nout, J.flags, err, S);
 }
 
+}  // namespace sbg
+#include "sbg_fused.cuh"
+namespace sbg {
+
 // ------------------------------------------------------------------------
 // launchers
 // ------------------------------------------------------------------------
@@ -1712,6 +1716,7 @@ cudaError_t set_kernel_attributes() {
 #define SBG_ATTR3S(n) if (e == cudaSuccess) e = col3s_attr<n>();
     SBG_COL3S_CASES(SBG_ATTR3S)
 #undef SBG_ATTR3S
+    if (e == cudaSuccess) e = fused_attr();
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     if (e == cudaSuccess)
@@ -1939,6 +1944,40 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
     KT_END(kt, KID_COL_INV, st);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
+}
+
+cudaError_t launch_fused(const JobDesc& J, int lgL, const LenPlan* lp, const uint2* tw_f, const uint2* tw_i,
+                         uint32_t* err, cudaStream_t st, KTimer* kt) {
+    ScaleArg sc;
+    for (int q = 0; q < SBG_NP; ++q) {
+        sc.w[q] = lp->scale[q].w;
+        sc.ws[q] = lp->scale[q].ws;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(SBG_NP, 1, 1);
+    cfg.blockDim = dim3(FU_T, 1, 1);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = SBG_NP;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaErrorInvalidValue;
+    KT_BEGIN(kt, KID_SMALL, st);
+    switch (lgL) {
+#define SBG_LAUNCH_FU(n)                                                     \
+    case n:                                                                  \
+        cfg.dynamicSmemBytes = sizeof(FusedSmem<n>);                         \
+        e = cudaLaunchKernelEx(&cfg, k_fused<n>, J, tw_f, tw_i, sc, err);    \
+        break;
+        SBG_FUSED_CASES(SBG_LAUNCH_FU)
+#undef SBG_LAUNCH_FU
+        default: break;
+    }
+    KT_END(kt, KID_SMALL, st);
+    return e;
 }
 
 int64_t crt_blocks(int64_t nout) { return (nout + 1 + CRT_BLK - 1) / CRT_BLK; }

@@ -38,17 +38,24 @@ struct RLog {
     static constexpr int v = (R == 2) ? 1 : (R == 4) ? 2 : (R == 8) ? 3 : (R == 16) ? 4 : 5;
 };
 
+// A twiddle table in global memory (read through L1) or staged in shared memory.
+struct SharedTw {
+    const uint2* p;
+};
+__device__ __forceinline__ uint2 tw_at(const uint2* t, int i) { return __ldg(t + i); }
+__device__ __forceinline__ uint2 tw_at(SharedTw t, int i) { return t.p[i]; }
+
 // forward DIF levels of one group (block size 2^lgM, stride st).  J0Z: the
 // caller's j0 is 0, so the butterflies at tin = 0 have the twiddle 1 and
 // skip the multiply (and the table load).
 // HZ: the upper half of the inputs is zero (see dif_regs2).
-template <int R, bool J0Z = false, bool HZ = false>
-__device__ __forceinline__ void dif_regs(uint32_t (&x)[R], const uint2* __restrict__ tw, int j0,
+template <int R, bool J0Z = false, bool HZ = false, typename TW>
+__device__ __forceinline__ void dif_regs(uint32_t (&x)[R], TW tw, int j0,
                                          int st, int lgM, uint32_t p) {
     if constexpr (HZ) {
 #pragma unroll
         for (int t = 0; t < R / 2; ++t) {
-            uint2 w = __ldg(&tw[tw_idx(lgM, j0 + st * t)]);
+            uint2 w = tw_at(tw, tw_idx(lgM, j0 + st * t));
             x[t + R / 2] = mul_shoup(x[t], w.x, w.y, p);
         }
     }
@@ -62,7 +69,7 @@ __device__ __forceinline__ void dif_regs(uint32_t (&x)[R], const uint2* __restri
                 bfly_triv(x[t], x[t + h], p);
                 continue;
             }
-            uint2 w = __ldg(&tw[tw_idx(lgM - l, j0 + st * tin)]);
+            uint2 w = tw_at(tw, tw_idx(lgM - l, j0 + st * tin));
             bfly_gs(x[t], x[t + h], w.x, w.y, p);
         }
     }
@@ -71,14 +78,14 @@ __device__ __forceinline__ void dif_regs(uint32_t (&x)[R], const uint2* __restri
 // two groups sharing (j0, st, lgM): one twiddle load serves both.  HZ: the
 // upper half of both groups' inputs is zero (a zero-padded operand), so the
 // first level is (u, 0) -> (u, u w): one multiply, no add or reduction.
-template <int R, bool J0Z = false, bool HZ = false>
+template <int R, bool J0Z = false, bool HZ = false, typename TW>
 __device__ __forceinline__ void dif_regs2(uint32_t (&x)[R], uint32_t (&y)[R],
-                                          const uint2* __restrict__ tw, int j0, int st, int lgM,
+                                          TW tw, int j0, int st, int lgM,
                                           uint32_t p) {
     if constexpr (HZ) {
 #pragma unroll
         for (int t = 0; t < R / 2; ++t) {
-            uint2 w = __ldg(&tw[tw_idx(lgM, j0 + st * t)]);
+            uint2 w = tw_at(tw, tw_idx(lgM, j0 + st * t));
             x[t + R / 2] = mul_shoup(x[t], w.x, w.y, p);
             y[t + R / 2] = mul_shoup(y[t], w.x, w.y, p);
         }
@@ -94,7 +101,7 @@ __device__ __forceinline__ void dif_regs2(uint32_t (&x)[R], uint32_t (&y)[R],
                 bfly_triv(y[t], y[t + h], p);
                 continue;
             }
-            uint2 w = __ldg(&tw[tw_idx(lgM - l, j0 + st * tin)]);
+            uint2 w = tw_at(tw, tw_idx(lgM - l, j0 + st * tin));
             bfly_gs(x[t], x[t + h], w.x, w.y, p);
             bfly_gs(y[t], y[t + h], w.x, w.y, p);
         }
@@ -102,8 +109,8 @@ __device__ __forceinline__ void dif_regs2(uint32_t (&x)[R], uint32_t (&y)[R],
 }
 
 // inverse: the forward group's levels in reverse, Cooley-Tukey with w^-1
-template <int R, bool J0Z = false>
-__device__ __forceinline__ void dit_regs(uint32_t (&x)[R], const uint2* __restrict__ twi, int j0,
+template <int R, bool J0Z = false, typename TW>
+__device__ __forceinline__ void dit_regs(uint32_t (&x)[R], TW twi, int j0,
                                          int st, int lgM, uint32_t p) {
     constexpr int r = RLog<R>::v;
 #pragma unroll
@@ -117,15 +124,15 @@ __device__ __forceinline__ void dit_regs(uint32_t (&x)[R], const uint2* __restri
                 bfly_triv(x[t], x[t + h], p);
                 continue;
             }
-            uint2 w = __ldg(&twi[tw_idx(lgM - l, j0 + st * tin)]);
+            uint2 w = tw_at(twi, tw_idx(lgM - l, j0 + st * tin));
             bfly_ct(x[t], x[t + h], w.x, w.y, p);
         }
     }
 }
 
-template <int R, bool J0Z = false>
+template <int R, bool J0Z = false, typename TW>
 __device__ __forceinline__ void dit_regs2(uint32_t (&x)[R], uint32_t (&y)[R],
-                                          const uint2* __restrict__ twi, int j0, int st, int lgM,
+                                          TW twi, int j0, int st, int lgM,
                                           uint32_t p) {
     constexpr int r = RLog<R>::v;
 #pragma unroll
@@ -140,7 +147,7 @@ __device__ __forceinline__ void dit_regs2(uint32_t (&x)[R], uint32_t (&y)[R],
                 bfly_triv(y[t], y[t + h], p);
                 continue;
             }
-            uint2 w = __ldg(&twi[tw_idx(lgM - l, j0 + st * tin)]);
+            uint2 w = tw_at(twi, tw_idx(lgM - l, j0 + st * tin));
             bfly_ct(x[t], x[t + h], w.x, w.y, p);
             bfly_ct(y[t], y[t + h], w.x, w.y, p);
         }
