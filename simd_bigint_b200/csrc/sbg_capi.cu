@@ -157,7 +157,8 @@ static int run_conv(sbg_ctx* c, uint64_t* rp, const uint64_t* ap, int64_t an, co
     st = ensure_ws(c, ws_words(lgL, sq), carry_flag_words(nout));
     if (st) return st;
     const LenPlan* lp = &c->plans[lgL];
-    CK(launch_conv(ap, an, bp, bn, sq, lgL, lp, c->tw_f, c->tw_i, c->ws, c->stream, c->timer, b_ready));
+    CK(launch_conv(ap, an, bp, bn, sq, lgL, lp, c->tw_f, c->tw_i, c->ws, c->flags,
+                   (int64_t)carry_flag_words(nout), c->stream, c->timer, b_ready));
     CK(launch_crt_carry(c->ws, lgL, lp, cmin, cmax, off, rp, nout, c->flags, c->err, c->stream,
                         c->timer));
     // the split forward columns (b_ready on the four-step path) are two launches
@@ -265,7 +266,7 @@ static int batch_launch(sbg_batch* b, KTimer* kt) {
         if (pers && persist_code(cl.lgL)) continue;
         cudaStream_t st = b->aux[k++ % SBG_BATCH_STREAMS];
         CK(launch_batch_class(cl.djobs, cl.njobs, cl.lgL, &c->plans[cl.lgL], c->tw_f, c->tw_i,
-                              cl.max_nout, cl.flags, cl.flag_words, c->err, st, kt));
+                              cl.max_nout, cl.flags, cl.flag_words, c->err, st, kt, b->classes.size() == 1));
     }
     if (pers) {
         CK(cudaMemsetAsync(b->d_state, 0, b->state_words * sizeof(uint32_t), c->stream));
@@ -543,7 +544,7 @@ int enqueue_products(sbg_ctx* c, const sbg_job* jobs, int64_t count, uint32_t* e
         const Cls& k = cls[i];
         CK(launch_batch_class((const JobDesc*)dd + k.first, k.njobs, k.lgL, &c->plans[k.lgL], c->tw_f,
                               c->tw_i, max_nout[k.lgL], k.flags, k.flag_words, err ? err : c->err,
-                              c->aux[i % SBG_AUX_STREAMS], c->timer));
+                              c->aux[i % SBG_AUX_STREAMS], c->timer, cls.size() == 1));
         c->launches += class_launches(k.lgL);
     }
     for (int k = 0; k < nst; ++k) {

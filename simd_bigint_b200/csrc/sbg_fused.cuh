@@ -87,6 +87,7 @@ __device__ __forceinline__ void fused_body(int q, const JobDesc& J, const uint2*
 #pragma unroll
     for (int i = 0; i < (int)sizeof(CrtConst) / 4; i += 16) touch |= reinterpret_cast<const uint32_t*>(&c_crt)[i];
     asm volatile("" ::"r"(touch));
+    pdl_enter();                               // operands and results only from here on
     // first pass: limbs -> residues -> four levels
     const int op = tid / NG, gid = tid & (NG - 1);
     const bool in_op = op < (J.sq ? 1 : 2);

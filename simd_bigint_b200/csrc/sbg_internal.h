@@ -13,6 +13,58 @@
 
 namespace sbg {
 
+#ifdef __CUDACC__
+// Programmatic dependent launch.  A kernel launched with the attribute may
+// start while the one before it on its stream still runs; pdl_wait() returns
+// when that one has finished and its writes are visible, pdl_launch() lets the
+// next one start.  Every such kernel waits first and only then lets the next
+// one start, so whatever was queued before the previous kernel is complete at
+// a kernel's entry: tables may be read ahead of the wait, a predecessor's
+// results and the caller's operands only after it, and nothing is written
+// before it.  Without the attribute both are no-ops.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+// wait, then let the next kernel in
+__device__ __forceinline__ void pdl_enter() {
+    pdl_wait();
+    pdl_launch();
+}
+// <<<blocks, threads, smem, st>>>, in clusters of `cluster` CTAs, with the
+// attribute if `pdl`.  It is used where launch gaps count and nothing else runs
+// beside the chain: single products of up to SBG_PDL_POINTS transform points
+// (16384 x 16384 limbs: 29.5 -> 20.3 us a call with it and without the flags'
+// memset, 333333 x 77777: 65.5 -> 59.6; at 2^24 x 2^20, where the waiting CTAs
+// only take room, 2605 -> 2674) and product lists of one length class (a
+// reciprocal of 100000 limbs: 1348 -> 1217 us).  In a batch of several
+// classes the waiting CTAs of one stream keep other streams' kernels out (1024
+// products: 1352 -> 1363 us), so there it is off.
+#define SBG_PDL_POINTS ((int64_t)1 << 20)
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kern)(KArgs...), bool pdl, int64_t blocks, int threads, size_t smem, int cluster,
+                              cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks, 1, 1);
+    cfg.blockDim = dim3((unsigned)threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = (unsigned)cluster;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+#endif
+
 // Transform lengths are identified by a code: c <= SBG_MAX_LG is L = 2^c,
 // c = SBG_CODE3 + k is L = 3 * 2^k (four-step only, k >= SBG_THREE_MIN_LG),
 // chosen when it is the smaller of the two lengths that hold a product.
@@ -184,14 +236,15 @@ cudaError_t gen_len_tables(LenPlan* lp, cudaStream_t st);
 
 // Whole product through the transform pipeline.  Workspace `ws` must hold
 // ws_words(code) u32.  `err` is a device word that receives sticky error bits.
-// Every `lgL` below is a length code.
+// Every `lgL` below is a length code.  Transforms of more than 2^12 points
+// clear flags[0 .. nflags), the words of the carry scan that follows.
 size_t ws_words(int lgL, int sq);
 // b_ready (optional): an event the second operand's arrival is recorded
 // on; the first operand's forward transform does not wait for it.
 cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_t bn, int sq,
                         int lgL, const LenPlan* lp, const uint2* tw_f, const uint2* tw_i,
-                        uint32_t* ws, cudaStream_t st, KTimer* kt = nullptr,
-                        cudaEvent_t b_ready = nullptr);
+                        uint32_t* ws, uint32_t* flags, int64_t nflags, cudaStream_t st,
+                        KTimer* kt = nullptr, cudaEvent_t b_ready = nullptr);
 // CRT + carry of residues R (5 x L u32) into out[0..nout): out[m] = limb (m + off)
 // of sum_{cmin <= j <= cmax} c_j * 2^(64 j).
 cudaError_t launch_crt_carry(const uint32_t* R, int lgL, const LenPlan* lp, int64_t cmin,
@@ -227,11 +280,12 @@ cudaError_t launch_fused(const JobDesc& J, int lgL, const LenPlan* lp, const uin
                          uint32_t* err, cudaStream_t st, KTimer* kt = nullptr);
 int64_t crt_blocks(int64_t nout);
 // All stages of one size class of the batch engine (every job of length
-// 2^lgL); `flags` holds flag_words zero-initialised words, job regions inside.
+// 2^lgL); `flags` holds flag_words words, job regions inside (cleared here).
+// alone: no other class runs beside it.
 cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const LenPlan* lp,
                                const uint2* tw_f, const uint2* tw_i, int64_t max_nout,
                                uint32_t* flags, size_t flag_words, uint32_t* err,
-                               cudaStream_t st, KTimer* kt = nullptr);
+                               cudaStream_t st, KTimer* kt = nullptr, bool alone = false);
 
 
 // ---- the context (C ABI opaque type), shared by the library's TUs ----

@@ -111,8 +111,12 @@ __global__ void __launch_bounds__(256) k_small(const uint64_t* __restrict__ a, i
 // batched: one CTA per (job, prime); every job of the launch has length 2^lgL
 __global__ void __launch_bounds__(256) k_small_b(const JobDesc* __restrict__ jobs, int lgL,
                                                  const uint2* __restrict__ twf,
-                                                 const uint2* __restrict__ twi, ScaleArg sc) {
+                                                 const uint2* __restrict__ twi, ScaleArg sc,
+                                                 uint32_t* flags, int64_t nflags) {
+    pdl_enter();
     const JobDesc& J = jobs[blockIdx.x / SBG_NP];
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nflags) flags[i] = 0;                // the carry scan's ticket and flags
     small_body(blockIdx.x % SBG_NP, J.a, J.an, J.b, J.bn, J.sq, lgL, twf, twi, sc, J.ws);
 }
 
@@ -623,6 +627,7 @@ __global__ void __launch_bounds__(COL_THREADS, COL_FWD_MINB) k_col_fwd(const uin
                                                     const uint2* __restrict__ twf,
                                                     uint32_t* __restrict__ YA,
                                                     uint32_t* __restrict__ YB, int nops) {
+    pdl_enter();
     constexpr int LGC = col_lgc(LGN1);
     constexpr int NTILES = col_ntiles(LGN1);
     const int slab = blockIdx.x & ((1 << LGC) - 1);
@@ -637,6 +642,7 @@ __global__ void __launch_bounds__(COL_THREADS, COL_FWD_MINB) k_col_fwd(const uin
 template <int LGN1>
 __global__ void __launch_bounds__(COL_THREADS, COL_FWD_MINB) k_col_fwd_b(const JobDesc* __restrict__ jobs,
                                                       const uint2* __restrict__ twf) {
+    pdl_enter();
     constexpr int LGC = col_lgc(LGN1);
     constexpr int NTILES = col_ntiles(LGN1);
     constexpr int PER_JOB = (SBG_NP * 2 * NTILES) << LGC;
@@ -676,6 +682,7 @@ __device__ __forceinline__ void col_inv_body(int q, int tile, int slab, uint32_t
 template <int LGN1>
 __global__ void __launch_bounds__(COL_THREADS, COL_MINB) k_col_inv(uint32_t* __restrict__ YA,
                                                     const uint2* __restrict__ twi) {
+    pdl_enter();
     constexpr int LGC = col_lgc(LGN1);
     const int slab = blockIdx.x & ((1 << LGC) - 1);
     const int rest = blockIdx.x >> LGC;
@@ -685,6 +692,7 @@ __global__ void __launch_bounds__(COL_THREADS, COL_MINB) k_col_inv(uint32_t* __r
 template <int LGN1>
 __global__ void __launch_bounds__(COL_THREADS, COL_MINB) k_col_inv_b(const JobDesc* __restrict__ jobs,
                                                       const uint2* __restrict__ twi) {
+    pdl_enter();
     constexpr int LGC = col_lgc(LGN1);
     constexpr int NTILES = col_ntiles(LGN1);
     constexpr int PER_JOB = (SBG_NP * NTILES) << LGC;
@@ -949,6 +957,7 @@ __global__ void __launch_bounds__(COL_THREADS, COL3_FWD_MINB) k_col3s_fwd(const 
                                                                    const uint2* __restrict__ twf, Radix3Arg r3,
                                                                    uint32_t* __restrict__ YA,
                                                                    uint32_t* __restrict__ YB) {
+    pdl_enter();
     constexpr int NTILES = col3s_ntiles(M3);
     const int q = blockIdx.x % SBG_NP;
     const int rest = blockIdx.x / SBG_NP;
@@ -958,6 +967,7 @@ __global__ void __launch_bounds__(COL_THREADS, COL3_FWD_MINB) k_col3s_fwd(const 
 template <int M3>
 __global__ void __launch_bounds__(COL_THREADS, COL3_FWD_MINB) k_col3s_fwd_b(const JobDesc* __restrict__ jobs,
                                                                      const uint2* __restrict__ twf, Radix3Arg r3) {
+    pdl_enter();
     constexpr int NTILES = col3s_ntiles(M3);
     constexpr int PER_JOB = SBG_NP * 2 * NTILES;
     constexpr size_t L = (size_t)3 << (M3 + SBG_ROW_LG);
@@ -973,12 +983,14 @@ __global__ void __launch_bounds__(COL_THREADS, COL3_FWD_MINB) k_col3s_fwd_b(cons
 template <int M3>
 __global__ void __launch_bounds__(COL_THREADS, COL_MINB) k_col3s_inv(uint32_t* __restrict__ YA,
                                                                    const uint2* __restrict__ twi, Radix3Arg r3) {
+    pdl_enter();
     col3s_inv_body<M3>(blockIdx.x % SBG_NP, blockIdx.x / SBG_NP, YA, twi, r3);
 }
 
 template <int M3>
 __global__ void __launch_bounds__(COL_THREADS, COL_MINB) k_col3s_inv_b(const JobDesc* __restrict__ jobs,
                                                                      const uint2* __restrict__ twi, Radix3Arg r3) {
+    pdl_enter();
     constexpr int NTILES = col3s_ntiles(M3);
     constexpr int PER_JOB = SBG_NP * NTILES;
     const JobDesc& J = jobs[blockIdx.x / PER_JOB];
@@ -993,6 +1005,7 @@ __global__ void __launch_bounds__(COL_THREADS, COL3_FWD_MINB) k_col3_fwd(const u
                                                                   const uint2* __restrict__ twf, Radix3Arg r3,
                                                                   uint32_t* __restrict__ YA,
                                                                   uint32_t* __restrict__ YB) {
+    pdl_enter();
     constexpr int C = col3_csize(M3);
     constexpr int NTILES = col3_ntiles(M3);
     const int slab = blockIdx.x % C;
@@ -1005,6 +1018,7 @@ __global__ void __launch_bounds__(COL_THREADS, COL3_FWD_MINB) k_col3_fwd(const u
 template <int M3>
 __global__ void __launch_bounds__(COL_THREADS, COL3_FWD_MINB) k_col3_fwd_b(const JobDesc* __restrict__ jobs,
                                                                     const uint2* __restrict__ twf, Radix3Arg r3) {
+    pdl_enter();
     constexpr int C = col3_csize(M3);
     constexpr int NTILES = col3_ntiles(M3);
     constexpr int PER_JOB = SBG_NP * 2 * NTILES * C;
@@ -1023,6 +1037,7 @@ __global__ void __launch_bounds__(COL_THREADS, COL3_FWD_MINB) k_col3_fwd_b(const
 template <int M3>
 __global__ void __launch_bounds__(COL_THREADS, COL_MINB) k_col3_inv(uint32_t* __restrict__ YA,
                                                                   const uint2* __restrict__ twi, Radix3Arg r3) {
+    pdl_enter();
     constexpr int C = col3_csize(M3);
     const int slab = blockIdx.x % C;
     const int rest = blockIdx.x / C;
@@ -1032,6 +1047,7 @@ __global__ void __launch_bounds__(COL_THREADS, COL_MINB) k_col3_inv(uint32_t* __
 template <int M3>
 __global__ void __launch_bounds__(COL_THREADS, COL_MINB) k_col3_inv_b(const JobDesc* __restrict__ jobs,
                                                                     const uint2* __restrict__ twi, Radix3Arg r3) {
+    pdl_enter();
     constexpr int C = col3_csize(M3);
     constexpr int NTILES = col3_ntiles(M3);
     constexpr int PER_JOB = SBG_NP * NTILES * C;
@@ -1187,11 +1203,20 @@ __device__ __forceinline__ void row_body(int q, int row, uint32_t* __restrict__ 
     }
 }
 
+// The carry scan that follows needs its ticket and flags zero; the row
+// kernel, which has more threads than there are flags, clears them.
+__device__ __forceinline__ void clear_flags(uint32_t* flags, int64_t n) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) flags[i] = 0;
+}
+
 __global__ void __launch_bounds__(256, ROW_MINB) k_row12(uint32_t* __restrict__ YA,
                                                   const uint32_t* __restrict__ YB, int sq,
                                                   int lgN1, int m3, FsTables fsf, FsTables fsi,
                                                   ScaleArg sc, const uint2* __restrict__ twf,
-                                                  const uint2* __restrict__ twi) {
+                                                  const uint2* __restrict__ twi, uint32_t* flags, int64_t nflags) {
+    pdl_enter();
+    clear_flags(flags, nflags);
     __shared__ RowSmem S;
     const int n1 = m3 >= 0 ? 3 << m3 : 1 << lgN1;
     const int q = blockIdx.x / n1;
@@ -1202,7 +1227,9 @@ __global__ void __launch_bounds__(256, ROW_MINB) k_row12(uint32_t* __restrict__ 
 __global__ void __launch_bounds__(256, ROW_MINB) k_row12_b(const JobDesc* __restrict__ jobs, int lgN1,
                                                     int m3, FsTables fsf, FsTables fsi, ScaleArg sc,
                                                     const uint2* __restrict__ twf,
-                                                    const uint2* __restrict__ twi) {
+                                                    const uint2* __restrict__ twi, uint32_t* flags, int64_t nflags) {
+    pdl_enter();
+    clear_flags(flags, nflags);
     const int n1 = m3 >= 0 ? 3 << m3 : 1 << lgN1;
     const int per_job = SBG_NP * n1;
     const JobDesc& J = jobs[blockIdx.x / per_job];
@@ -1600,6 +1627,7 @@ __global__ void __launch_bounds__(CRT_T, CRT_MINB) k_crt_carry(const uint32_t* _
                                                      int64_t cmin, int64_t cmax, int64_t off,
                                                      uint64_t* __restrict__ out, int64_t nout,
                                                      uint32_t* flags, uint32_t* err) {
+    pdl_enter();
     __shared__ uint32_t s_bid;
     if (threadIdx.x == 0) s_bid = atomicAdd(&flags[0], 1u);
     __syncthreads();
@@ -1620,6 +1648,7 @@ __global__ void __launch_bounds__(CRT_T, CRT_MINB) k_crt_carry_s(const uint32_t*
                                                        int64_t cmin, int64_t cmax, int64_t off,
                                                        uint64_t* __restrict__ out, int64_t nout,
                                                        uint32_t* flags, uint32_t* err) {
+    pdl_enter();
     __shared__ uint32_t s_bid;
     if (threadIdx.x == 0) s_bid = atomicAdd(&flags[0], 1u);
     __syncthreads();
@@ -1631,6 +1660,7 @@ __global__ void __launch_bounds__(CRT_T, CRT_MINB) k_crt_carry_s(const uint32_t*
 // launch); each takes a ticket on its own job's counter, surplus ones exit.
 __global__ void __launch_bounds__(CRT_T, CRT_MINB) k_crt_carry_b(const JobDesc* __restrict__ jobs, int64_t L,
                                                        int blocks_per_job, uint32_t* err) {
+    pdl_enter();
     __shared__ uint32_t s_bid;
     const JobDesc& J = jobs[blockIdx.x / blocks_per_job];
     if (threadIdx.x == 0) s_bid = atomicAdd(&J.flags[0], 1u);
@@ -1794,26 +1824,14 @@ size_t ws_words(int lgL, int sq) {
 // Column kernels: COL_THREADS threads, dynamic shared memory, and a
 // cluster of `cluster` CTAs when a column spans several slabs.
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_colx(void (*kern)(KArgs...), int64_t blocks, int smem, int cluster,
+static cudaError_t launch_colx(void (*kern)(KArgs...), bool pdl, int64_t blocks, int smem, int cluster,
                                cudaStream_t st, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks, 1, 1);
-    cfg.blockDim = dim3(COL_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)cluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = cluster > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
+    return launch_pdl(kern, pdl, blocks, COL_THREADS, (size_t)smem, cluster, st, args...);
 }
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_col(void (*kern)(KArgs...), int lgN1, int64_t blocks, cudaStream_t st,
+static cudaError_t launch_col(void (*kern)(KArgs...), bool pdl, int lgN1, int64_t blocks, cudaStream_t st,
                               Args... args) {
-    return launch_colx(kern, blocks, col_smem_bytes(lgN1), 1 << col_lgc(lgN1), st, args...);
+    return launch_colx(kern, pdl, blocks, col_smem_bytes(lgN1), 1 << col_lgc(lgN1), st, args...);
 }
 
 
@@ -1829,8 +1847,10 @@ static Radix3Arg radix3_arg(const LenPlan* lp, bool inverse) {
 
 cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_t bn, int sq,
                         int lgL, const LenPlan* lp, const uint2* tw_f, const uint2* tw_i,
-                        uint32_t* ws, cudaStream_t st, KTimer* kt, cudaEvent_t b_ready) {
+                        uint32_t* ws, uint32_t* flags, int64_t nflags, cudaStream_t st, KTimer* kt,
+                        cudaEvent_t b_ready) {
     const size_t L = (size_t)code_len(lgL);
+    const bool pdl = (int64_t)L <= SBG_PDL_POINTS;
     // the first operand's forward columns may start before the second
     // operand has arrived only on the power-of-two four-step path
     const bool split = b_ready && !sq && lgL > SBG_SMALL_MAX_LG && lp->m3 < 0;
@@ -1864,14 +1884,14 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
         switch (m3) {
 #define SBG_LAUNCH_F3S(n)                                                                          \
     case n:                                                                                        \
-        e = launch_colx(k_col3s_fwd<n>, (int64_t)nops * col3s_ntiles(n) * SBG_NP, col3s_smem_bytes(n), 1, \
+        e = launch_colx(k_col3s_fwd<n>, pdl, (int64_t)nops * col3s_ntiles(n) * SBG_NP, col3s_smem_bytes(n), 1, \
                         st, a, an, b, bn, tw_f, r3f, YA, YB);                                       \
         break;
             SBG_COL3S_CASES(SBG_LAUNCH_F3S)
 #undef SBG_LAUNCH_F3S
 #define SBG_LAUNCH_F3(n)                                                                          \
     case n:                                                                                       \
-        e = launch_colx(k_col3_fwd<n>, (int64_t)nops * col3_ntiles(n) * SBG_NP * col3_csize(n),    \
+        e = launch_colx(k_col3_fwd<n>, pdl, (int64_t)nops * col3_ntiles(n) * SBG_NP * col3_csize(n),    \
                         col3_smem_bytes(n), col3_csize(n), st, a, an, b, bn, tw_f, r3f, YA, YB); \
         break;
             SBG_COL3_CASES(SBG_LAUNCH_F3)
@@ -1881,21 +1901,22 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
         KT_END(kt, KID_COL_FWD, st);
         if (e != cudaSuccess) return e;
         KT_BEGIN(kt, KID_ROW, st);
-        k_row12<<<(3 << m3) * SBG_NP, 256, 0, st>>>(YA, YB, sq, 0, m3, fsf, fsi, sc, tw_f, tw_i);
+        e = launch_pdl(k_row12, pdl, (int64_t)(3 << m3) * SBG_NP, 256, 0, 1, st, YA, YB, sq, 0, m3, fsf, fsi, sc, tw_f, tw_i,
+                       flags, nflags);
         KT_END(kt, KID_ROW, st);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if (e != cudaSuccess) return e;
         KT_BEGIN(kt, KID_COL_INV, st);
         switch (m3) {
 #define SBG_LAUNCH_I3S(n)                                                                          \
     case n:                                                                                        \
-        e = launch_colx(k_col3s_inv<n>, (int64_t)col3s_ntiles(n) * SBG_NP, col3s_smem_bytes(n), 1, st, YA, \
+        e = launch_colx(k_col3s_inv<n>, pdl, (int64_t)col3s_ntiles(n) * SBG_NP, col3s_smem_bytes(n), 1, st, YA, \
                         tw_i, r3i);                                                                 \
         break;
             SBG_COL3S_CASES(SBG_LAUNCH_I3S)
 #undef SBG_LAUNCH_I3S
 #define SBG_LAUNCH_I3(n)                                                                             \
     case n:                                                                                          \
-        e = launch_colx(k_col3_inv<n>, (int64_t)col3_ntiles(n) * SBG_NP * col3_csize(n),               \
+        e = launch_colx(k_col3_inv<n>, pdl, (int64_t)col3_ntiles(n) * SBG_NP * col3_csize(n),               \
                         col3_smem_bytes(n), col3_csize(n), st, YA, tw_i, r3i);                        \
         break;
             SBG_COL3_CASES(SBG_LAUNCH_I3)
@@ -1912,12 +1933,12 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
 #define SBG_LAUNCH_F(n)                                                                          \
     case n:                                                                                      \
         if (split) {                                                                             \
-            e = launch_col(k_col_fwd<n>, n, col_blocks, st, a, an, a, an, tw_f, YA, YA, 1);        \
+            e = launch_col(k_col_fwd<n>, pdl, n, col_blocks, st, a, an, a, an, tw_f, YA, YA, 1);        \
             if (e == cudaSuccess) e = cudaStreamWaitEvent(st, b_ready, 0);                        \
             if (e == cudaSuccess)                                                                \
-                e = launch_col(k_col_fwd<n>, n, col_blocks, st, b, bn, b, bn, tw_f, YB, YB, 1);    \
+                e = launch_col(k_col_fwd<n>, pdl, n, col_blocks, st, b, bn, b, bn, tw_f, YB, YB, 1);    \
         } else {                                                                                 \
-            e = launch_col(k_col_fwd<n>, n, nops * col_blocks, st, a, an, b, bn, tw_f, YA, YB, nops); \
+            e = launch_col(k_col_fwd<n>, pdl, n, nops * col_blocks, st, a, an, b, bn, tw_f, YA, YB, nops); \
         }                                                                                        \
         break;
         SBG_COL_CASES(SBG_LAUNCH_F)
@@ -1929,14 +1950,14 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     KT_BEGIN(kt, KID_ROW, st);
-    k_row12<<<(1 << lgN1) * SBG_NP, 256, 0, st>>>(YA, YB, sq, lgN1, -1, fsf, fsi, sc, tw_f, tw_i);
+    e = launch_pdl(k_row12, pdl, (int64_t)SBG_NP << lgN1, 256, 0, 1, st, YA, YB, sq, lgN1, -1, fsf, fsi, sc, tw_f, tw_i, flags,
+                   nflags);
     KT_END(kt, KID_ROW, st);
-    e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     KT_BEGIN(kt, KID_COL_INV, st);
     switch (lgN1) {
 #define SBG_LAUNCH_I(n) \
-    case n: e = launch_col(k_col_inv<n>, n, col_blocks, st, YA, tw_i); break;
+    case n: e = launch_col(k_col_inv<n>, pdl, n, col_blocks, st, YA, tw_i); break;
         SBG_COL_CASES(SBG_LAUNCH_I)
 #undef SBG_LAUNCH_I
         default: return cudaErrorInvalidValue;
@@ -1953,24 +1974,12 @@ cudaError_t launch_fused(const JobDesc& J, int lgL, const LenPlan* lp, const uin
         sc.w[q] = lp->scale[q].w;
         sc.ws[q] = lp->scale[q].ws;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(SBG_NP, 1, 1);
-    cfg.blockDim = dim3(FU_T, 1, 1);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = SBG_NP;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     cudaError_t e = cudaErrorInvalidValue;
     KT_BEGIN(kt, KID_SMALL, st);
     switch (lgL) {
-#define SBG_LAUNCH_FU(n)                                                     \
-    case n:                                                                  \
-        cfg.dynamicSmemBytes = sizeof(FusedSmem<n>);                         \
-        e = cudaLaunchKernelEx(&cfg, k_fused<n>, J, tw_f, tw_i, sc, err);    \
+#define SBG_LAUNCH_FU(n)                                                                                        \
+    case n:                                                                                                     \
+        e = launch_pdl(k_fused<n>, true, SBG_NP, FU_T, sizeof(FusedSmem<n>), SBG_NP, st, J, tw_f, tw_i, sc, err);     \
         break;
         SBG_FUSED_CASES(SBG_LAUNCH_FU)
 #undef SBG_LAUNCH_FU
@@ -1985,7 +1994,7 @@ int64_t crt_blocks(int64_t nout) { return (nout + 1 + CRT_BLK - 1) / CRT_BLK; }
 cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const LenPlan* lp,
                                const uint2* tw_f, const uint2* tw_i, int64_t max_nout,
                                uint32_t* flags, size_t flag_words, uint32_t* err,
-                               cudaStream_t st, KTimer* kt) {
+                               cudaStream_t st, KTimer* kt, bool alone) {
     if (njobs <= 0) return cudaSuccess;
     if (lgL == SBG_CODE_SCHOOL) {
         KT_BEGIN(kt, KID_BATCH, st);
@@ -1998,12 +2007,14 @@ cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const L
         sc.w[q] = lp->scale[q].w;
         sc.ws[q] = lp->scale[q].ws;
     }
-    cudaError_t e = cudaMemsetAsync(flags, 0, flag_words * sizeof(uint32_t), st);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
+    const bool pdl = alone && (int64_t)njobs * code_len(lgL) <= SBG_PDL_POINTS;
     KT_BEGIN(kt, KID_BATCH, st);
     if (lgL <= SBG_SMALL_MAX_LG) {
         size_t smem = (size_t)2 * padded_len(1 << lgL) * 4;
-        k_small_b<<<njobs * SBG_NP, 256, smem, st>>>(djobs, lgL, tw_f, tw_i, sc);
+        e = launch_pdl(k_small_b, pdl, (int64_t)njobs * SBG_NP, 256, smem, 1, st, djobs, lgL, tw_f, tw_i, sc, flags,
+                       (int64_t)flag_words);
+        if (e != cudaSuccess) return e;
     } else if (lp->m3 >= 0) {
         const int m3 = lp->m3;
         FsTables fsf{lp->fs_lo_f, lp->fs_hi_f, lp->hi_n};
@@ -2012,14 +2023,14 @@ cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const L
         switch (m3) {
 #define SBG_LAUNCH_FB3S(n)                                                                              \
     case n:                                                                                             \
-        e = launch_colx(k_col3s_fwd_b<n>, (int64_t)njobs * 2 * col3s_ntiles(n) * SBG_NP, col3s_smem_bytes(n), \
+        e = launch_colx(k_col3s_fwd_b<n>, pdl, (int64_t)njobs * 2 * col3s_ntiles(n) * SBG_NP, col3s_smem_bytes(n), \
                         1, st, djobs, tw_f, r3f);                                                        \
         break;
             SBG_COL3S_CASES(SBG_LAUNCH_FB3S)
 #undef SBG_LAUNCH_FB3S
 #define SBG_LAUNCH_FB3(n)                                                                       \
     case n:                                                                                     \
-        e = launch_colx(k_col3_fwd_b<n>, (int64_t)njobs * 2 * col3_ntiles(n) * SBG_NP * col3_csize(n), \
+        e = launch_colx(k_col3_fwd_b<n>, pdl, (int64_t)njobs * 2 * col3_ntiles(n) * SBG_NP * col3_csize(n), \
                         col3_smem_bytes(n), col3_csize(n), st, djobs, tw_f, r3f);                \
         break;
             SBG_COL3_CASES(SBG_LAUNCH_FB3)
@@ -2027,18 +2038,20 @@ cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const L
             default: return cudaErrorInvalidValue;
         }
         if (e != cudaSuccess) return e;
-        k_row12_b<<<njobs * SBG_NP * (3 << m3), 256, 0, st>>>(djobs, 0, m3, fsf, fsi, sc, tw_f, tw_i);
+        e = launch_pdl(k_row12_b, pdl, (int64_t)njobs * SBG_NP * (3 << m3), 256, 0, 1, st, djobs, 0, m3, fsf, fsi, sc,
+                       tw_f, tw_i, flags, (int64_t)flag_words);
+        if (e != cudaSuccess) return e;
         switch (m3) {
 #define SBG_LAUNCH_IB3S(n)                                                                           \
     case n:                                                                                          \
-        e = launch_colx(k_col3s_inv_b<n>, (int64_t)njobs * col3s_ntiles(n) * SBG_NP, col3s_smem_bytes(n), \
+        e = launch_colx(k_col3s_inv_b<n>, pdl, (int64_t)njobs * col3s_ntiles(n) * SBG_NP, col3s_smem_bytes(n), \
                         1, st, djobs, tw_i, r3i);                                                     \
         break;
             SBG_COL3S_CASES(SBG_LAUNCH_IB3S)
 #undef SBG_LAUNCH_IB3S
 #define SBG_LAUNCH_IB3(n)                                                                     \
     case n:                                                                                   \
-        e = launch_colx(k_col3_inv_b<n>, (int64_t)njobs * col3_ntiles(n) * SBG_NP * col3_csize(n), \
+        e = launch_colx(k_col3_inv_b<n>, pdl, (int64_t)njobs * col3_ntiles(n) * SBG_NP * col3_csize(n), \
                         col3_smem_bytes(n), col3_csize(n), st, djobs, tw_i, r3i);              \
         break;
             SBG_COL3_CASES(SBG_LAUNCH_IB3)
@@ -2053,16 +2066,18 @@ cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const L
         const int64_t col_blocks = ((int64_t)njobs * col_ntiles(lgN1) * SBG_NP) << col_lgc(lgN1);
         switch (lgN1) {
 #define SBG_LAUNCH_FB(n) \
-    case n: e = launch_col(k_col_fwd_b<n>, n, 2 * col_blocks, st, djobs, tw_f); break;
+    case n: e = launch_col(k_col_fwd_b<n>, pdl, n, 2 * col_blocks, st, djobs, tw_f); break;
             SBG_COL_CASES(SBG_LAUNCH_FB)
 #undef SBG_LAUNCH_FB
             default: return cudaErrorInvalidValue;
         }
         if (e != cudaSuccess) return e;
-        k_row12_b<<<(njobs * SBG_NP) << lgN1, 256, 0, st>>>(djobs, lgN1, -1, fsf, fsi, sc, tw_f, tw_i);
+        e = launch_pdl(k_row12_b, pdl, (int64_t)(njobs * SBG_NP) << lgN1, 256, 0, 1, st, djobs, lgN1, -1, fsf, fsi, sc,
+                       tw_f, tw_i, flags, (int64_t)flag_words);
+        if (e != cudaSuccess) return e;
         switch (lgN1) {
 #define SBG_LAUNCH_IB(n) \
-    case n: e = launch_col(k_col_inv_b<n>, n, col_blocks, st, djobs, tw_i); break;
+    case n: e = launch_col(k_col_inv_b<n>, pdl, n, col_blocks, st, djobs, tw_i); break;
             SBG_COL_CASES(SBG_LAUNCH_IB)
 #undef SBG_LAUNCH_IB
             default: return cudaErrorInvalidValue;
@@ -2070,9 +2085,9 @@ cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const L
         if (e != cudaSuccess) return e;
     }
     const int bpj = (int)crt_blocks(max_nout);
-    k_crt_carry_b<<<njobs * bpj, CRT_T, 0, st>>>(djobs, code_len(lgL), bpj, err);
+    e = launch_pdl(k_crt_carry_b, pdl, (int64_t)njobs * bpj, CRT_T, 0, 1, st, djobs, code_len(lgL), bpj, err);
     KT_END(kt, KID_BATCH, st);
-    return cudaGetLastError();
+    return e;
 }
 
 // ticket + one flag per block + the error word's slot, for either block
@@ -2093,15 +2108,15 @@ cudaError_t launch_crt_carry(const uint32_t* R, int lgL, const LenPlan* lp, int6
     const bool shortp = nout <= CRT_SHORT_MAX;
     const int64_t blk = shortp ? CRT_SHORT_BLK : CRT_BLK;
     int64_t nblk = (nout + 1 + blk - 1) / blk;
-    cudaError_t e = cudaMemsetAsync(flags, 0, (1 + nblk) * sizeof(uint32_t), st);
+    cudaError_t e = cudaSuccess;
+    if (lgL <= SBG_SMALL_MAX_LG)         // longer transforms: the row kernel has cleared them
+        e = cudaMemsetAsync(flags, 0, (1 + nblk) * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     KT_BEGIN(kt, KID_CRT, st);
-    if (shortp)
-        k_crt_carry_s<<<(unsigned)nblk, CRT_T, 0, st>>>(R, code_len(lgL), cmin, cmax, off, out, nout, flags, err);
-    else
-        k_crt_carry<<<(unsigned)nblk, CRT_T, 0, st>>>(R, code_len(lgL), cmin, cmax, off, out, nout, flags, err);
+    e = launch_pdl(shortp ? k_crt_carry_s : k_crt_carry, code_len(lgL) <= SBG_PDL_POINTS, nblk, CRT_T, 0, 1, st, R, code_len(lgL), cmin, cmax, off, out,
+                   nout, flags, err);
     KT_END(kt, KID_CRT, st);
-    return cudaGetLastError();
+    return e;
 }
 
 }  // namespace sbg

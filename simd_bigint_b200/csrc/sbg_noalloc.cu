@@ -151,7 +151,7 @@ extern "C" int sbg_mul_noalloc(uint64_t* rp, const uint64_t* ap, int64_t an, con
     uint32_t* res = d->scratch;
     uint32_t* flags = d->scratch + SBG_NOALLOC_RES_WORDS;
     uint32_t* err = flags + SBG_NOALLOC_FLAG_WORDS;
-    if (launch_conv(ap, an, bp, bn, 0, lgL, &lp, d->tw_f, d->tw_i, res, st) != cudaSuccess)
+    if (launch_conv(ap, an, bp, bn, 0, lgL, &lp, d->tw_f, d->tw_i, res, flags, 0, st) != cudaSuccess)
         return SBG_ECUDA;
     if (launch_crt_carry(res, lgL, &lp, 0, an + bn - 2, 0, rp, an + bn, flags, err, st) !=
         cudaSuccess)

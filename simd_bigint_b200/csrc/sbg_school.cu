@@ -46,6 +46,7 @@ __global__ void __launch_bounds__(SCHOOL_T) k_school(const uint64_t* __restrict_
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int step = wid % SCHOOL_STEPS, part = wid / SCHOOL_STEPS;
     const int n = an + bn;
+    pdl_enter();
     for (int i = tid; i < 3 * MAX; i += SCHOOL_T) sb[i] = i >= MAX && i < MAX + bn ? __ldg(&b[i - MAX]) : 0;
     if (tid < an) sa[tid] = __ldg(&a[tid]);
     if (tid < 3) {
@@ -121,8 +122,7 @@ __global__ void __launch_bounds__(32 * SCHOOL_WARPS) k_school_b(const JobDesc* _
 cudaError_t launch_school(const uint64_t* a, int64_t an, const uint64_t* b, int64_t bn,
                           uint64_t* out, cudaStream_t st) {
     if (an <= 0 || bn <= 0 || an + bn > SBG_SCHOOL_MAX) return cudaErrorInvalidValue;
-    k_school<<<1, SCHOOL_T, 0, st>>>(a, (int)an, b, (int)bn, out);
-    return cudaGetLastError();
+    return launch_pdl(k_school, true, 1, SCHOOL_T, 0, 1, st, a, (int)an, b, (int)bn, out);
 }
 
 cudaError_t launch_school_batch(const JobDesc* djobs, int njobs, cudaStream_t st) {
