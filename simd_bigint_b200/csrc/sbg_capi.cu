@@ -133,7 +133,8 @@ static int ensure_ws(sbg_ctx* c, size_t words, size_t flag_words) {
 // sum_{cmin <= j <= cmax} c_j 2^(64 j) where c = a * b (cyclic length 2^lgL).
 static int run_conv(sbg_ctx* c, uint64_t* rp, const uint64_t* ap, int64_t an, const uint64_t* bp,
                     int64_t bn, int sq, int lgL, int64_t cmin, int64_t cmax, int64_t off,
-                    int64_t nout, cudaEvent_t b_ready = nullptr) {
+                    int64_t nout, cudaEvent_t b_ready = nullptr, uint32_t* err = nullptr) {
+    if (!err) err = c->err;
     if (lgL > SBG_NCODES || code_len(lgL) > ((int64_t)1 << SBG_MAX_LG)) return SBG_EBAND;
     int st = ensure_plan(c, lgL);
     if (st) return st;
@@ -150,7 +151,7 @@ static int run_conv(sbg_ctx* c, uint64_t* rp, const uint64_t* ap, int64_t an, co
         J.off = off;
         J.nout = nout;
         J.sq = sq;
-        CK(launch_fused(J, lgL, &c->plans[lgL], c->tw_f, c->tw_i, c->err, c->stream, c->timer));
+        CK(launch_fused(J, lgL, &c->plans[lgL], c->tw_f, c->tw_i, err, c->stream, c->timer));
         c->launches += 1;
         return SBG_OK;
     }
@@ -159,7 +160,7 @@ static int run_conv(sbg_ctx* c, uint64_t* rp, const uint64_t* ap, int64_t an, co
     const LenPlan* lp = &c->plans[lgL];
     CK(launch_conv(ap, an, bp, bn, sq, lgL, lp, c->tw_f, c->tw_i, c->ws, c->flags,
                    (int64_t)carry_flag_words(nout), c->stream, c->timer, b_ready));
-    CK(launch_crt_carry(c->ws, lgL, lp, cmin, cmax, off, rp, nout, c->flags, c->err, c->stream,
+    CK(launch_crt_carry(c->ws, lgL, lp, cmin, cmax, off, rp, nout, c->flags, err, c->stream,
                         c->timer));
     // the split forward columns (b_ready on the four-step path) are two launches
     c->launches += class_launches(lgL) + ((b_ready && !sq && lgL > SBG_SMALL_MAX_LG && lp->m3 < 0) ? 1 : 0);
@@ -463,6 +464,20 @@ void UploadRing::release() {
 
 int enqueue_products(sbg_ctx* c, const sbg_job* jobs, int64_t count, uint32_t* err) {
     if (count <= 0) return SBG_OK;
+    if (count == 1) {
+        // one product needs no descriptor list and no forked stream: the
+        // single-product kernels take it as arguments (the upload, two events
+        // and the batched kernels' indirection cost it about 15 us)
+        const sbg_job& j = jobs[0];
+        int lgL, sq;
+        int64_t cmin, cmax, off, nout;
+        int st = job_shape(j, c->len3_mask, &lgL, &cmin, &cmax, &off, &nout, &sq);
+        if (st) return st;
+        const uint64_t* bp = sq ? j.ap : j.bp;
+        const int64_t bn = sq ? j.an : j.bn;
+        if (lgL == SBG_CODE_SCHOOL) return run_school(c, j.rp, j.ap, j.an, bp, bn);
+        return run_conv(c, j.rp, j.ap, j.an, bp, bn, sq, lgL, cmin, cmax, off, nout, nullptr, err);
+    }
     std::vector<JobDesc> by_lg[SBG_NCODES + 1];
     int64_t max_nout[SBG_NCODES + 1] = {};
     for (int64_t i = 0; i < count; ++i) {
@@ -537,14 +552,15 @@ int enqueue_products(sbg_ctx* c, const sbg_job* jobs, int64_t count, uint32_t* e
     void* dd = nullptr;
     int st = c->ring.push(all.data(), all.size() * sizeof(JobDesc), c->stream, &dd);
     if (st) return st;
-    CK(cudaEventRecord(c->fork, c->stream));
-    const int nst = std::min<int>(SBG_AUX_STREAMS, (int)cls.size());
+    // a list of one class stays on the context's stream
+    const int nst = cls.size() == 1 ? 0 : std::min<int>(SBG_AUX_STREAMS, (int)cls.size());
+    if (nst) CK(cudaEventRecord(c->fork, c->stream));
     for (int k = 0; k < nst; ++k) CK(cudaStreamWaitEvent(c->aux[k], c->fork, 0));
     for (size_t i = 0; i < cls.size(); ++i) {
         const Cls& k = cls[i];
         CK(launch_batch_class((const JobDesc*)dd + k.first, k.njobs, k.lgL, &c->plans[k.lgL], c->tw_f,
                               c->tw_i, max_nout[k.lgL], k.flags, k.flag_words, err ? err : c->err,
-                              c->aux[i % SBG_AUX_STREAMS], c->timer, cls.size() == 1));
+                              nst ? c->aux[i % SBG_AUX_STREAMS] : c->stream, c->timer, !nst));
         c->launches += class_launches(k.lgL);
     }
     for (int k = 0; k < nst; ++k) {

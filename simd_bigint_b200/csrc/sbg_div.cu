@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 #include "../../include/simd_bigint_b200.h"
@@ -46,6 +47,10 @@ namespace cg = cooperative_groups;
 // rounds, where few divisions remain -- spread over DIV_CL SMs.
 #define DIV_CL 8
 #define DIV_CL_MIN_N 32768
+// Where at most DIV_CL_FEW divisions are in a step, clusters of them fit on
+// the device side by side and shorter ones are spread as well.
+#define DIV_CL_FEW 16
+#define DIV_CL_FEW_MIN_N 6144
 
 // The CTA group of one division: its rank, a barrier over all of its
 // threads (release / acquire: global and shared memory written before it
@@ -565,13 +570,18 @@ __device__ bool warp_divrem(const uint64_t* __restrict__ D, int m, NF nlimb, int
 
 // exact base case of the Newton recursion: X = floor((B^2m - 1) / A), m+1
 // limbs (top limb 1), m <= SBG_DIV_BASE; one warp per divisor
-__global__ void __launch_bounds__(32 * WDIV_WARPS) k_recip_base(const uint64_t* const* A, const int64_t* m,
-                                                              uint64_t* const* X, int count, uint32_t* err) {
+struct RecipBase {
+    const uint64_t* A;      // m limbs
+    uint64_t* X;            // m+1 limbs out
+    int64_t m;
+};
+__global__ void __launch_bounds__(32 * WDIV_WARPS) k_recip_base(const RecipBase* b, int count, uint32_t* err) {
+    pdl_enter();
     const int idx = blockIdx.x * WDIV_WARPS + (threadIdx.x >> 5);
     if (idx >= count) return;
-    const int n = (int)m[idx];
-    uint64_t* q = X[idx];
-    const bool ok = warp_divrem(A[idx], n, [](int64_t) { return ~0ull; }, 2 * (int64_t)n, q, nullptr);
+    const int n = (int)b[idx].m;
+    uint64_t* q = b[idx].X;
+    const bool ok = warp_divrem(b[idx].A, n, [](int64_t) { return ~0ull; }, 2 * (int64_t)n, q, nullptr);
     __syncwarp();
     if ((threadIdx.x & 31) == 0 && (!ok || q[n] != 1)) atomicOr(err, 8u);
 }
@@ -610,6 +620,7 @@ __global__ void __launch_bounds__(32 * WDIV_WARPS) k_divrem_warp(const WarpDiv* 
 
 template <int CL>
 __global__ void __launch_bounds__(DIV_T) k_recip_wrap(const RecipStep* st, uint32_t* err) {
+    pdl_enter();
     __shared__ long long s_slot[2];
     Grp<CL> grp(s_slot);
     const RecipStep S = st[blockIdx.x / CL];
@@ -652,6 +663,7 @@ __global__ void __launch_bounds__(DIV_T) k_recip_wrap(const RecipStep* st, uint3
 // step 1: correct X_h while T >= B^(n+h); T_m = limbs l..n of B^(n+h) - T
 template <int CL>
 __global__ void __launch_bounds__(DIV_T) k_recip_step1(const RecipStep* st, uint32_t* err) {
+    pdl_enter();
     __shared__ long long s_slot[2];
     Grp<CL> grp(s_slot);
     const RecipStep S = st[blockIdx.x / CL];
@@ -725,6 +737,7 @@ __global__ void __launch_bounds__(DIV_T) k_recip_step1(const RecipStep* st, uint
 // step 2: X = X_h * B^l + floor(U / B^(2h-l))
 template <int CL>
 __global__ void __launch_bounds__(DIV_T) k_recip_step2(const RecipStep* st) {
+    pdl_enter();
     __shared__ long long s_slot[2];
     Grp<CL> grp(s_slot);
     const RecipStep S = st[blockIdx.x / CL];
@@ -745,6 +758,7 @@ __global__ void __launch_bounds__(DIV_T) k_recip_step2(const RecipStep* st) {
 // Q0 = N_hi + floor(P / B^n), P = N_hi * V (2n limbs)
 template <int CL>
 __global__ void __launch_bounds__(DIV_T) k_div_q0(const DivFix* df) {
+    pdl_enter();
     __shared__ long long s_slot[2];
     Grp<CL> grp(s_slot);
     const DivFix F = df[blockIdx.x / CL];
@@ -761,6 +775,7 @@ __global__ void __launch_bounds__(DIV_T) k_div_q0(const DivFix* df) {
 // N - C mod (B^L - 1), N folded to L limbs, C = Q0 D mod (B^L - 1).
 template <int CL>
 __global__ void __launch_bounds__(DIV_T) k_div_fix(const DivFix* df, uint32_t* err) {
+    pdl_enter();
     __shared__ long long s_slot[2];
     Grp<CL> grp(s_slot);
     const DivFix F = df[blockIdx.x / CL];
@@ -833,6 +848,7 @@ __global__ void __launch_bounds__(DIV_T) k_div_fix(const DivFix* df, uint32_t* e
 // computed from P = D * X (2n+1 limbs): R = complement of P's low n+1 limbs
 template <int CL>
 __global__ void __launch_bounds__(DIV_T) k_recip_final(const DivFix* df, uint32_t* err) {
+    pdl_enter();
     __shared__ long long s_slot[2];
     Grp<CL> grp(s_slot);
     const DivFix F = df[blockIdx.x / CL];
@@ -909,6 +925,7 @@ struct CopyDesc {
 };
 #define COPY_BPD 8          // blocks per descriptor
 __global__ void __launch_bounds__(256) k_copy_pad(const CopyDesc* d) {
+    pdl_enter();
     const CopyDesc D = d[blockIdx.x / COPY_BPD];
     const int64_t stride = (int64_t)COPY_BPD * blockDim.x;
     for (int64_t i = (int64_t)(blockIdx.x % COPY_BPD) * blockDim.x + threadIdx.x; i < D.n_dst; i += stride)
@@ -921,9 +938,9 @@ static int copy_batch(sbg_ctx* c, const std::vector<CopyDesc>& cp) {
         CopyDesc* dd = nullptr;
         int rc = upload(c, part, &dd);
         if (rc) return rc;
-        k_copy_pad<<<(unsigned)(cnt * COPY_BPD), 256, 0, c->stream>>>(dd);
+        if (launch_pdl(k_copy_pad, true, (int64_t)cnt * COPY_BPD, 256, 0, 1, c->stream, (const CopyDesc*)dd) != cudaSuccess)
+            return SBG_ECUDA;
         c->launches += 1;
-        if (cudaGetLastError() != cudaSuccess) return SBG_ECUDA;
     }
     return SBG_OK;
 }
@@ -934,25 +951,15 @@ template <class D, class... KA, class... A>
 static int launch_lin(sbg_ctx* c, void (*k1)(const D*, KA...), void (*kc)(const D*, KA...), const D* d,
                       int ns, int nb, A... a) {
     if (ns > 0) {
-        k1<<<ns, DIV_T, 0, c->stream>>>(d, a...);
+        if (launch_pdl(k1, true, ns, DIV_T, 0, 1, c->stream, d, a...) != cudaSuccess) return SBG_ECUDA;
         c->launches += 1;
     }
     if (nb > 0) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)nb * DIV_CL);
-        cfg.blockDim = dim3(DIV_T);
-        cfg.stream = c->stream;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = DIV_CL;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        if (cudaLaunchKernelEx(&cfg, kc, d + ns, a...) != cudaSuccess) return SBG_ECUDA;
+        if (launch_pdl(kc, true, (int64_t)nb * DIV_CL, DIV_T, 0, DIV_CL, c->stream, d + ns, a...) != cudaSuccess)
+            return SBG_ECUDA;
         c->launches += 1;
     }
-    return cudaGetLastError() == cudaSuccess ? SBG_OK : SBG_ECUDA;
+    return SBG_OK;
 }
 
 // Reciprocals (and optionally quotients) of every instance; all scratch set.
@@ -966,29 +973,22 @@ static int div_core(sbg_ctx* c, std::vector<DivInst>& v, uint32_t* err, bool quo
         maxd = std::max(maxd, (int)d.sz.size() - 1);
     }
     int rc = SBG_OK;
-    // base case: X[cur] of every instance
-    {
-        std::vector<const uint64_t*> A;
-        std::vector<int64_t> m;
-        std::vector<uint64_t*> X;
-        for (auto& d : v) {
-            const int64_t mb = d.sz.back();
-            A.push_back(d.D + (d.n - mb));
-            m.push_back(mb);
-            X.push_back(d.X[(d.sz.size() - 1) & 1]);
-        }
-        const uint64_t** dA = nullptr;
-        int64_t* dm = nullptr;
-        uint64_t** dX = nullptr;
-        if ((rc = upload(c, A, &dA)) || (rc = upload(c, m, &dm)) || (rc = upload(c, X, &dX))) return rc;
-        k_recip_base<<<((int)v.size() + WDIV_WARPS - 1) / WDIV_WARPS, 32 * WDIV_WARPS, 0, st>>>(
-            dA, dm, dX, (int)v.size(), err);
-        c->launches += 1;
-        if (cudaGetLastError() != cudaSuccess) return SBG_ECUDA;
-    }
-    for (int r = 1; r <= maxd && !rc; ++r) {
-        std::vector<sbg_job> jt, ju;
-        std::vector<RecipStep> steps, big;       // single-CTA divisions, clustered ones
+    // Every round's descriptors are known beforehand: the base cases' and all
+    // rounds' steps go up in one piece.
+    struct Round {
+        std::vector<sbg_job> jt, ju;             // the two products of the divisions in it
+        size_t first = 0;                        // its steps: single-CTA divisions, clustered ones
+        int ns = 0, nb = 0;
+    };
+    std::vector<Round> rounds((size_t)maxd);
+    std::vector<RecipStep> steps;
+    for (int r = 1; r <= maxd; ++r) {
+        Round& R = rounds[(size_t)r - 1];
+        std::vector<RecipStep> big;
+        R.first = steps.size();
+        int live = 0;
+        for (auto& d : v) live += (int)d.sz.size() - 1 >= r;
+        const int64_t cl_min = live <= DIV_CL_FEW ? DIV_CL_FEW_MIN_N : DIV_CL_MIN_N;
         for (auto& d : v) {
             const int depth = (int)d.sz.size() - 1;
             if (depth < r) continue;
@@ -1009,30 +1009,46 @@ static int div_core(sbg_ctx* c, std::vector<DivInst>& v, uint32_t* err, bool quo
             if (code_len(cwrap) < code_len(cfull)) {
                 S.L = code_len(cwrap);
                 S.C = d.U;
-                jt.push_back(sbg_job{S.C, S.A, S.Xh, n, h + 1, SBG_JOB_CYCLIC, cwrap});
+                R.jt.push_back(sbg_job{S.C, S.A, S.Xh, n, h + 1, SBG_JOB_CYCLIC, cwrap});
             } else {
-                jt.push_back(sbg_job{S.T, S.A, S.Xh, n, h + 1, SBG_JOB_MUL, 0});
+                R.jt.push_back(sbg_job{S.T, S.A, S.Xh, n, h + 1, SBG_JOB_MUL, 0});
             }
-            (n >= DIV_CL_MIN_N ? big : steps).push_back(S);
-            ju.push_back(sbg_job{d.U, S.TM, S.Xh, h + 1, h + 1, SBG_JOB_MUL, 0});
+            (n >= cl_min ? big : steps).push_back(S);
+            R.ju.push_back(sbg_job{d.U, S.TM, S.Xh, h + 1, h + 1, SBG_JOB_MUL, 0});
         }
-        const int ns = (int)steps.size(), nb = (int)big.size();
-        if (ns + nb == 0) continue;
+        R.nb = (int)big.size();
+        R.ns = (int)(steps.size() - R.first);
         steps.insert(steps.end(), big.begin(), big.end());
-        RecipStep* dsteps = nullptr;
-        if ((rc = upload(c, steps, &dsteps))) break;
-        if ((rc = enqueue_products(c, jt.data(), (int64_t)jt.size(), err))) break;
-        if ((rc = launch_lin(c, k_recip_wrap<1>, k_recip_wrap<DIV_CL>, (const RecipStep*)dsteps, ns, nb, err)))
-            break;
-        if ((rc = launch_lin(c, k_recip_step1<1>, k_recip_step1<DIV_CL>, (const RecipStep*)dsteps, ns, nb, err)))
-            break;
-        if ((rc = enqueue_products(c, ju.data(), (int64_t)ju.size(), err))) break;
-        if ((rc = launch_lin(c, k_recip_step2<1>, k_recip_step2<DIV_CL>, (const RecipStep*)dsteps, ns, nb)))
-            break;
+    }
+    const size_t nbase = v.size() * sizeof(RecipBase), soff = (nbase + 15) & ~(size_t)15;
+    std::vector<uint8_t> desc(soff + steps.size() * sizeof(RecipStep));
+    for (size_t i = 0; i < v.size(); ++i) {
+        DivInst& d = v[i];
+        const int64_t mb = d.sz.back();
+        const RecipBase b{d.D + (d.n - mb), d.X[(d.sz.size() - 1) & 1], mb};
+        std::memcpy(desc.data() + i * sizeof(RecipBase), &b, sizeof(b));
+    }
+    if (!steps.empty()) std::memcpy(desc.data() + soff, steps.data(), steps.size() * sizeof(RecipStep));
+    uint8_t* ddesc = nullptr;
+    if ((rc = upload(c, desc, &ddesc))) return rc;
+    if (launch_pdl(k_recip_base, true, ((int64_t)v.size() + WDIV_WARPS - 1) / WDIV_WARPS, 32 * WDIV_WARPS, 0, 1, st,
+                   (const RecipBase*)ddesc, (int)v.size(), err) != cudaSuccess)
+        return SBG_ECUDA;
+    c->launches += 1;
+    for (int r = 1; r <= maxd && !rc; ++r) {
+        const Round& R = rounds[(size_t)r - 1];
+        if (R.ns + R.nb == 0) continue;
+        const RecipStep* ds = (const RecipStep*)(ddesc + soff) + R.first;
+        if ((rc = enqueue_products(c, R.jt.data(), (int64_t)R.jt.size(), err))) break;
+        if ((rc = launch_lin(c, k_recip_wrap<1>, k_recip_wrap<DIV_CL>, ds, R.ns, R.nb, err))) break;
+        if ((rc = launch_lin(c, k_recip_step1<1>, k_recip_step1<DIV_CL>, ds, R.ns, R.nb, err))) break;
+        if ((rc = enqueue_products(c, R.ju.data(), (int64_t)R.ju.size(), err))) break;
+        if ((rc = launch_lin(c, k_recip_step2<1>, k_recip_step2<DIV_CL>, ds, R.ns, R.nb))) break;
     }
     if (rc) return rc;
     // final stage: exact reciprocal, or quotient and remainder
     std::vector<DivFix> fx, fxb;             // single-CTA divisions, clustered ones
+    const int64_t cl_min = v.size() <= DIV_CL_FEW ? DIV_CL_FEW_MIN_N : DIV_CL_MIN_N;
     std::vector<sbg_job> jp;
     std::vector<CopyDesc> cpx;
     for (auto& d : v) {
@@ -1051,7 +1067,7 @@ static int div_core(sbg_ctx* c, std::vector<DivInst>& v, uint32_t* err, bool quo
         F.R = quotient ? d.Rout : d.Qout;
         F.Rw = d.Rw;
         F.n = d.n;
-        (d.n >= DIV_CL_MIN_N ? fxb : fx).push_back(F);
+        (d.n >= cl_min ? fxb : fx).push_back(F);
         uint64_t* X = d.X[0];
         if (quotient) {
             // P = N_hi * V, V = low n limbs of X
