@@ -275,6 +275,131 @@ __global__ void __launch_bounds__(FU_T, 1) k_fused(const __grid_constant__ JobDe
 
 #define SBG_FUSED_CASES(X) X(8) X(9) X(10) X(11) X(12)
 
+// ------------------------------------------------------------------------
+// The row kernel of few rows.  k_row12 runs both operands of a row on 256
+// threads, four CTAs per SM, its twiddles read through L1: the right form when
+// rows queue for the SMs, but a lone row takes it 28,000 clocks, most of them
+// spent waiting for twiddles that no other CTA has brought to L1.  Here a row
+// has 512 threads, an operand to each half, and its twiddles staged in shared
+// memory -- before the previous kernel of the chain is waited for, as the
+// tables are older than that.  Device time a launch: 14.5 -> 9.9 us for 10 to
+// 80 rows; with two such CTAs on an SM (160 rows: 17.3 us) k_row12
+// higher throughput wins (320 rows: both 17 us).
+// ------------------------------------------------------------------------
+#define ROWL_MAX 148
+struct RowlSmem {
+    uint32_t A[padded_len(ROW_N)];
+    uint32_t B[padded_len(ROW_N)];
+    uint2 twf[ROW_N];
+    uint2 twi[ROW_N];
+    uint2 f[16];                               // four-step twiddle steps, w_L^(256 k1 t)
+    uint2 i[16];                               // their inverses times the CRT scale
+};
+
+template <bool BATCH>
+__global__ void __launch_bounds__(FU_T, 2) k_rowl(uint32_t* __restrict__ YA, const uint32_t* __restrict__ YB, int sq,
+                                                  const JobDesc* __restrict__ jobs, int lgN1, int m3, FsTables fsf,
+                                                  FsTables fsi, ScaleArg sc, const uint2* __restrict__ twf,
+                                                  const uint2* __restrict__ twi, uint32_t* flags, int64_t nflags) {
+    extern __shared__ __align__(16) uint8_t fu_raw[];
+    RowlSmem& S = *reinterpret_cast<RowlSmem*>(fu_raw);
+    constexpr int LG = ROW_LG;
+    const int n1 = m3 >= 0 ? 3 << m3 : 1 << lgN1;
+    const int per_job = SBG_NP * n1;
+    const int r = BATCH ? blockIdx.x % per_job : blockIdx.x;
+    const int q = r / n1, row = r - q * n1;
+    const int tid = threadIdx.x, op = tid >> 8, gid = tid & 255;
+    const PrimeConst pc = c_pr[q];
+    const uint32_t p = pc.p;
+    for (int k = tid; k < ROW_N; k += FU_T) {
+        const int h = k >= ROW_N / 2;
+        const int e = 2 * (h ? k - ROW_N / 2 : k);
+        const uint2* src = (h ? twi : twf) + (size_t)q * SBG_TW_N + e;
+        const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared((h ? S.twi : S.twf) + e));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    const SharedTw sf{S.twf}, si{S.twi};
+    // four-step twiddles of this row, as in row_body
+    const uint32_t k1 = m3 >= 0 ? 3u * bitrev((uint32_t)row & ((1u << m3) - 1u), m3) + ((uint32_t)row >> m3)
+                                : bitrev((uint32_t)row, lgN1);
+    if (tid < 32) {
+        const uint32_t e = k1 * 256u * (uint32_t)(tid & 15);
+        const uint32_t v = tid < 16 ? fs_value(fsf, q, e, p) : mul_shoup(fs_value(fsi, q, e, p), sc.w[q], sc.ws[q], p);
+        (tid < 16 ? S.f : S.i)[tid & 15] = make_uint2(v, shoup_fast(v, pc));
+    }
+    const uint32_t eb = k1 * (uint32_t)gid;
+    const uint32_t bf = fs_value(fsf, q, eb, p), bfs = shoup_fast(bf, pc);
+    const uint32_t bi = fs_value(fsi, q, eb, p), bis = shoup_fast(bi, pc);
+    pdl_enter();
+    clear_flags(flags, nflags);
+    if (BATCH) {
+        const JobDesc& J = jobs[blockIdx.x / per_job];
+        YA = J.ws;
+        YB = J.ws + (size_t)SBG_NP * n1 * ROW_N;
+        sq = J.sq;
+    }
+    const size_t base = ((size_t)q * n1 + row) * ROW_N;
+    const bool on = op == 0 || !sq;
+    uint32_t x[16];
+    if (on) {
+        const uint32_t* src = (op ? YB : YA) + base + gid;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) x[t] = __ldcg(src + 256 * t);
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    uint32_t* buf = op ? S.B : S.A;
+    if (on) {
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            const uint2 s = S.f[t];
+            x[t] = mul_shoup(mul_shoup(x[t], s.x, s.y, p), bf, bfs, p);
+        }
+        dif_regs<16>(x, sf, gid, 256, LG, p);
+#pragma unroll
+        for (int t = 0; t < 16; ++t) buf[padded_at<8>(gid, t)] = x[t];
+    }
+    __syncthreads();
+    if (on) fused_pass<LG, 1, true>(buf, gid, sf, p);
+    __syncthreads();
+    if (op == 0) {
+        // last forward pass, product, first inverse pass
+        const int i0 = gid << 4;
+        uint32_t y[16];
+#pragma unroll
+        for (int t = 0; t < 16; ++t) x[t] = S.A[padded_at<0>(i0, t)];
+        if (sq) {
+            dif_regs<16, true>(x, sf, 0, 1, 4, p);
+#pragma unroll
+            for (int t = 0; t < 16; ++t) x[t] = mont_mul(x[t], x[t], p, pc.pinv);
+        } else {
+#pragma unroll
+            for (int t = 0; t < 16; ++t) y[t] = S.B[padded_at<0>(i0, t)];
+            dif_regs2<16, true>(x, y, sf, 0, 1, 4, p);
+#pragma unroll
+            for (int t = 0; t < 16; ++t) x[t] = mont_mul(x[t], y[t], p, pc.pinv);
+        }
+        dit_regs<16, true>(x, si, 0, 1, 4, p);
+#pragma unroll
+        for (int t = 0; t < 16; ++t) S.A[padded_at<0>(i0, t)] = x[t];
+    }
+    __syncthreads();
+    if (op == 0) fused_pass<LG, 1, false>(S.A, gid, si, p);
+    __syncthreads();
+    if (op == 0) {
+#pragma unroll
+        for (int t = 0; t < 16; ++t) x[t] = S.A[padded_at<8>(gid, t)];
+        dit_regs<16>(x, si, gid, 256, LG, p);
+        uint32_t* dst = YA + base + gid;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            const uint2 s = S.i[t];
+            dst[256 * t] = mul_shoup(mul_shoup(x[t], s.x, s.y, p), bi, bis, p);
+        }
+    }
+}
+
 static cudaError_t fused_attr() {
     cudaError_t e = cudaSuccess;
 #define SBG_FUSED_ATTR(n) \
@@ -282,6 +407,10 @@ static cudaError_t fused_attr() {
         e = cudaFuncSetAttribute(k_fused<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FusedSmem<n>));
     SBG_FUSED_CASES(SBG_FUSED_ATTR)
 #undef SBG_FUSED_ATTR
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_rowl<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowlSmem));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_rowl<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowlSmem));
     return e;
 }
 

@@ -1845,6 +1845,30 @@ static Radix3Arg radix3_arg(const LenPlan* lp, bool inverse) {
     return r;
 }
 
+// the row kernel: few rows take the form with more threads per row
+static cudaError_t launch_rows(uint32_t* YA, const uint32_t* YB, int sq, const LenPlan* lp, const ScaleArg& sc,
+                               const uint2* tw_f, const uint2* tw_i, uint32_t* flags, int64_t nflags, bool pdl,
+                               cudaStream_t st) {
+    const FsTables fsf{lp->fs_lo_f, lp->fs_hi_f, lp->hi_n}, fsi{lp->fs_lo_i, lp->fs_hi_i, lp->hi_n};
+    const int64_t rows = SBG_NP * (lp->L >> ROW_LG);
+    if (rows <= ROWL_MAX)
+        return launch_pdl(k_rowl<false>, pdl, rows, FU_T, sizeof(RowlSmem), 1, st, YA, YB, sq, (const JobDesc*)nullptr,
+                          lp->lgN1, lp->m3, fsf, fsi, sc, tw_f, tw_i, flags, nflags);
+    return launch_pdl(k_row12, pdl, rows, 256, 0, 1, st, YA, YB, sq, lp->lgN1, lp->m3, fsf, fsi, sc, tw_f, tw_i, flags,
+                      nflags);
+}
+static cudaError_t launch_rows_b(const JobDesc* djobs, int njobs, const LenPlan* lp, const ScaleArg& sc,
+                                 const uint2* tw_f, const uint2* tw_i, uint32_t* flags, int64_t nflags, bool alone,
+                                 bool pdl, cudaStream_t st) {
+    const FsTables fsf{lp->fs_lo_f, lp->fs_hi_f, lp->hi_n}, fsi{lp->fs_lo_i, lp->fs_hi_i, lp->hi_n};
+    const int64_t rows = SBG_NP * (lp->L >> ROW_LG) * njobs;
+    if (alone && rows <= ROWL_MAX)
+        return launch_pdl(k_rowl<true>, pdl, rows, FU_T, sizeof(RowlSmem), 1, st, (uint32_t*)nullptr,
+                          (const uint32_t*)nullptr, 0, djobs, lp->lgN1, lp->m3, fsf, fsi, sc, tw_f, tw_i, flags, nflags);
+    return launch_pdl(k_row12_b, pdl, rows, 256, 0, 1, st, djobs, lp->lgN1, lp->m3, fsf, fsi, sc, tw_f, tw_i, flags,
+                      nflags);
+}
+
 cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_t bn, int sq,
                         int lgL, const LenPlan* lp, const uint2* tw_f, const uint2* tw_i,
                         uint32_t* ws, uint32_t* flags, int64_t nflags, cudaStream_t st, KTimer* kt,
@@ -1874,8 +1898,6 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
     }
     const int lgN1 = lp->lgN1;   // rows: 2^lgN1 (or 3 * 2^m3), columns: 2^12
     const int m3 = lp->m3;
-    FsTables fsf{lp->fs_lo_f, lp->fs_hi_f, lp->hi_n};
-    FsTables fsi{lp->fs_lo_i, lp->fs_hi_i, lp->hi_n};
     const int nops = sq ? 1 : 2;
     cudaError_t e = cudaSuccess;
     if (m3 >= 0) {
@@ -1901,8 +1923,7 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
         KT_END(kt, KID_COL_FWD, st);
         if (e != cudaSuccess) return e;
         KT_BEGIN(kt, KID_ROW, st);
-        e = launch_pdl(k_row12, pdl, (int64_t)(3 << m3) * SBG_NP, 256, 0, 1, st, YA, YB, sq, 0, m3, fsf, fsi, sc, tw_f, tw_i,
-                       flags, nflags);
+        e = launch_rows(YA, YB, sq, lp, sc, tw_f, tw_i, flags, nflags, pdl, st);
         KT_END(kt, KID_ROW, st);
         if (e != cudaSuccess) return e;
         KT_BEGIN(kt, KID_COL_INV, st);
@@ -1950,8 +1971,7 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     KT_BEGIN(kt, KID_ROW, st);
-    e = launch_pdl(k_row12, pdl, (int64_t)SBG_NP << lgN1, 256, 0, 1, st, YA, YB, sq, lgN1, -1, fsf, fsi, sc, tw_f, tw_i, flags,
-                   nflags);
+    e = launch_rows(YA, YB, sq, lp, sc, tw_f, tw_i, flags, nflags, pdl, st);
     KT_END(kt, KID_ROW, st);
     if (e != cudaSuccess) return e;
     KT_BEGIN(kt, KID_COL_INV, st);
@@ -2017,8 +2037,6 @@ cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const L
         if (e != cudaSuccess) return e;
     } else if (lp->m3 >= 0) {
         const int m3 = lp->m3;
-        FsTables fsf{lp->fs_lo_f, lp->fs_hi_f, lp->hi_n};
-        FsTables fsi{lp->fs_lo_i, lp->fs_hi_i, lp->hi_n};
         const Radix3Arg r3f = radix3_arg(lp, false), r3i = radix3_arg(lp, true);
         switch (m3) {
 #define SBG_LAUNCH_FB3S(n)                                                                              \
@@ -2038,8 +2056,7 @@ cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const L
             default: return cudaErrorInvalidValue;
         }
         if (e != cudaSuccess) return e;
-        e = launch_pdl(k_row12_b, pdl, (int64_t)njobs * SBG_NP * (3 << m3), 256, 0, 1, st, djobs, 0, m3, fsf, fsi, sc,
-                       tw_f, tw_i, flags, (int64_t)flag_words);
+        e = launch_rows_b(djobs, njobs, lp, sc, tw_f, tw_i, flags, (int64_t)flag_words, alone, pdl, st);
         if (e != cudaSuccess) return e;
         switch (m3) {
 #define SBG_LAUNCH_IB3S(n)                                                                           \
@@ -2061,8 +2078,6 @@ cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const L
         if (e != cudaSuccess) return e;
     } else {
         const int lgN1 = lp->lgN1;
-        FsTables fsf{lp->fs_lo_f, lp->fs_hi_f, lp->hi_n};
-        FsTables fsi{lp->fs_lo_i, lp->fs_hi_i, lp->hi_n};
         const int64_t col_blocks = ((int64_t)njobs * col_ntiles(lgN1) * SBG_NP) << col_lgc(lgN1);
         switch (lgN1) {
 #define SBG_LAUNCH_FB(n) \
@@ -2072,8 +2087,7 @@ cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const L
             default: return cudaErrorInvalidValue;
         }
         if (e != cudaSuccess) return e;
-        e = launch_pdl(k_row12_b, pdl, (int64_t)(njobs * SBG_NP) << lgN1, 256, 0, 1, st, djobs, lgN1, -1, fsf, fsi, sc,
-                       tw_f, tw_i, flags, (int64_t)flag_words);
+        e = launch_rows_b(djobs, njobs, lp, sc, tw_f, tw_i, flags, (int64_t)flag_words, alone, pdl, st);
         if (e != cudaSuccess) return e;
         switch (lgN1) {
 #define SBG_LAUNCH_IB(n) \
