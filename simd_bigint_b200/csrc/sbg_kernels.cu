@@ -1639,10 +1639,13 @@ __global__ void __launch_bounds__(CRT_T, CRT_MINB) k_crt_carry(const uint32_t* _
 // block), four times the blocks of k_crt_carry, so a short carry scan is
 // spread over more SMs (16384 x 16384 limbs: 14.7 -> 10.3 us); long ones
 // keep four steps, which fetch and compose fewer neighbour terms per limb.
+// The line is where 4096-limb blocks fill the SMs once: a product of 411,110
+// limbs takes 59.1 us with them and 55.5 with short ones, 800,000: 89.5 and
+// 87.9, 1,200,000: 147.9 and 149.0.
 #define CRT_SHORT_NSTEP 1
 #define CRT_SHORT_BLK ((CRT_T / 32) * 32 * CRT_V * CRT_SHORT_NSTEP)
 #ifndef CRT_SHORT_MAX
-#define CRT_SHORT_MAX (1 << 17)                 // product limbs up to which the short scan runs
+#define CRT_SHORT_MAX (3 << 18)                 // product limbs up to which the short scan runs
 #endif
 __global__ void __launch_bounds__(CRT_T, CRT_MINB) k_crt_carry_s(const uint32_t* __restrict__ R, int64_t L,
                                                        int64_t cmin, int64_t cmax, int64_t off,
