@@ -12,29 +12,35 @@
 // ballots, the cluster's from the (generate, propagate) bits of all its
 // warps.  Nothing goes through global memory between the limbs and the
 // product, and no flag is waited for.
-// What bounds it is the chain of passes on five SMs (20,000 clocks at 2^12
-// points, the SMs issuing 44% of them), so it is the single product's path;
-// batches fill the device with one CTA per prime and a separate carry scan.
-// 1500 x 1500 limbs, device time a call back to back: 30.7 us with the
-// transforms, the flags' memset and the carry scan as three launches, 12.3 us.
+// What bounds it is the chain of passes (20,000 clocks at 2^12 points, the
+// five SMs issuing 44% of them).  1500 x 1500 limbs, device time a call back
+// to back: 30.7 us with the transforms, the flags' memset and the carry scan
+// as three launches, 9.4 us.  A batch's classes run it too, one cluster per
+// job, with as many threads as the length has radix-16 groups: 128 divisions
+// 5.58 -> 5.30 ms, 1024 mixed products 1.352 -> 1.335 ms (640 CTAs of 2^8,
+// 2^10 and 2^12 points: 12 to 16, 16 and 40 us against 28, 36 and 67 us with
+// one CTA per prime and a carry scan).
 // Shorter transforms (2^4 .. 2^7, tiny middle products) keep those launches.
 #pragma once
 
 namespace sbg {
 
-#define FU_T 512
+#define FU_T 512                               // threads at 2^12 points, and of the row kernel below
+// threads at 2^LG points: a radix-16 group of either operand each
+__host__ __device__ constexpr int fu_threads(int lg) { return lg <= 9 ? 64 : 1 << (lg - 3); }
 #define FU_V 2                                 // limbs per thread in the carry phase
 
 template <int LG>
 struct FusedSmem {
+    static constexpr int FU_NW = fu_threads(LG) / 32;      // warps
     uint32_t A[padded_len(1 << LG)];
     uint32_t B[padded_len(1 << LG)];
     uint2 twf[1 << LG];
     uint2 twi[1 << LG];
-    ulonglong2 xlo[FU_T / 32][2];              // limbs of each warp's last two lanes
-    uint64_t xmid[FU_T / 32][2];
-    uint2 xhi[FU_T / 32][2];
-    uint32_t warp[FU_T / 32];                  // (G, P) of this CTA's warps
+    ulonglong2 xlo[FU_NW][2];              // limbs of each warp's last two lanes
+    uint64_t xmid[FU_NW][2];
+    uint2 xhi[FU_NW][2];
+    uint32_t warp[FU_NW];                  // (G, P) of this CTA's warps
 };
 
 __device__ __forceinline__ uint32_t dsmem_ld(uint32_t a) {
@@ -66,6 +72,7 @@ __device__ __forceinline__ void fused_body(int q, const JobDesc& J, const uint2*
     extern __shared__ __align__(16) uint8_t fu_raw[];
     FusedSmem<LG>& S = *reinterpret_cast<FusedSmem<LG>*>(fu_raw);
     constexpr int L = 1 << LG, NP = num_passes(LG), NG = L / 16;     // radix-16 groups per operand
+    constexpr int T = fu_threads(LG), FU_NW = T / 32;
     static_assert(NP == 2 || NP == 3, "two or three passes");
     constexpr unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -73,7 +80,7 @@ __device__ __forceinline__ void fused_body(int q, const JobDesc& J, const uint2*
     const uint32_t p = pc.p;
 
     // twiddles of every size up to L: 16-byte asynchronous copies
-    for (int i = tid; i < L; i += FU_T) {
+    for (int i = tid; i < L; i += T) {
         const int h = i >= L / 2;
         const int e = 2 * (h ? i - L / 2 : i);
         const uint2* src = (h ? twi : twf) + (size_t)q * SBG_TW_N + e;
@@ -121,7 +128,7 @@ __device__ __forceinline__ void fused_body(int q, const JobDesc& J, const uint2*
     // last forward pass, product times the CRT scale, first inverse pass
     {
         constexpr int K = NP - 1, r = prl(LG, K), R = 1 << r;
-        for (int g = tid; g < L / R; g += FU_T) {
+        for (int g = tid; g < L / R; g += T) {
             const int i0 = g << r;
             uint32_t x[R], y[R];
 #pragma unroll
@@ -236,16 +243,17 @@ __device__ __forceinline__ void fused_body(int q, const JobDesc& J, const uint2*
     }
     cluster_barrier<true>();                   // all warps' (G, P) are in shared memory
     // the carry into this warp: over the CTAs below, then this CTA's warps
+    constexpr uint32_t NWM = (1u << FU_NW) - 1u;
     uint32_t v[SBG_NP], cin = 0, cw = 0;
 #pragma unroll
     for (int k = 0; k < SBG_NP; ++k)
-        v[k] = k <= q && lane < FU_T / 32 ? dsmem_ld(dsmem_addr(S.warp, k) + 4 * lane) : 2u;
+        v[k] = k <= q && lane < FU_NW ? dsmem_ld(dsmem_addr(S.warp, k) + 4 * lane) : 2u;
 #pragma unroll
     for (int k = 0; k < SBG_NP; ++k) {
-        const uint32_t g = __ballot_sync(FULL, v[k] & 1u) & 0xffffu, pr = __ballot_sync(FULL, v[k] & 2u) & 0xffffu;
+        const uint32_t g = __ballot_sync(FULL, v[k] & 1u) & NWM, pr = __ballot_sync(FULL, v[k] & 2u) & NWM;
         const uint32_t sum = pr + ((g << 1) | cin);
         if (k == q) cw = (sum ^ pr) >> wid;
-        cin = ((sum >> (FU_T / 32)) | (g >> (FU_T / 32 - 1))) & 1u;
+        cin = ((sum >> (FU_NW)) | (g >> (FU_NW - 1))) & 1u;
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");     // peers' memory is read
     if (on) {
@@ -268,9 +276,18 @@ __device__ __forceinline__ void fused_body(int q, const JobDesc& J, const uint2*
 }
 
 template <int LG>
-__global__ void __launch_bounds__(FU_T, 1) k_fused(const __grid_constant__ JobDesc J, const uint2* __restrict__ twf,
+__global__ void __launch_bounds__(fu_threads(LG), 1) k_fused(const __grid_constant__ JobDesc J, const uint2* __restrict__ twf,
                                                    const uint2* __restrict__ twi, ScaleArg sc, uint32_t* err) {
     fused_body<LG>(blockIdx.x, J, twf, twi, sc.w[blockIdx.x], sc.ws[blockIdx.x], err);
+}
+
+// batched: one cluster per job
+template <int LG>
+__global__ void __launch_bounds__(fu_threads(LG), 1024 / fu_threads(LG))
+    k_fused_b(const JobDesc* __restrict__ jobs, const uint2* __restrict__ twf, const uint2* __restrict__ twi, ScaleArg sc,
+              uint32_t* err) {
+    const int q = blockIdx.x % SBG_NP;
+    fused_body<LG>(q, jobs[blockIdx.x / SBG_NP], twf, twi, sc.w[q], sc.ws[q], err);
 }
 
 #define SBG_FUSED_CASES(X) X(8) X(9) X(10) X(11) X(12)
@@ -404,7 +421,9 @@ static cudaError_t fused_attr() {
     cudaError_t e = cudaSuccess;
 #define SBG_FUSED_ATTR(n) \
     if (e == cudaSuccess) \
-        e = cudaFuncSetAttribute(k_fused<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FusedSmem<n>));
+        e = cudaFuncSetAttribute(k_fused<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FusedSmem<n>)); \
+    if (e == cudaSuccess) \
+        e = cudaFuncSetAttribute(k_fused_b<n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FusedSmem<n>));
     SBG_FUSED_CASES(SBG_FUSED_ATTR)
 #undef SBG_FUSED_ATTR
     if (e == cudaSuccess)

@@ -372,9 +372,11 @@ struct UploadRing {
 #define SBG_SMALL_MAX_LG 12
 
 // kernel launches of one product (or one length class of a batch): the
-// fused single-CTA transform or the three four-step transforms, then CRT+carry
+// whole short product, or the single-CTA transform or the three four-step
+// transforms, then CRT+carry
 inline int class_launches(int lgL) {
-    return lgL == SBG_CODE_SCHOOL ? 1 : (lgL <= SBG_SMALL_MAX_LG ? 2 : 4);
+    if (lgL == SBG_CODE_SCHOOL || (lgL >= SBG_FUSED_MIN_LG && lgL <= SBG_SMALL_MAX_LG)) return 1;
+    return lgL <= SBG_SMALL_MAX_LG ? 2 : 4;
 }
 // codes in the order batches launch them: longest transforms first
 inline int64_t code_order_key(int c) { return code_len(c); }

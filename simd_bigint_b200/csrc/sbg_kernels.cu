@@ -2002,7 +2002,7 @@ cudaError_t launch_fused(const JobDesc& J, int lgL, const LenPlan* lp, const uin
     switch (lgL) {
 #define SBG_LAUNCH_FU(n)                                                                                        \
     case n:                                                                                                     \
-        e = launch_pdl(k_fused<n>, true, SBG_NP, FU_T, sizeof(FusedSmem<n>), SBG_NP, st, J, tw_f, tw_i, sc, err);     \
+        e = launch_pdl(k_fused<n>, true, SBG_NP, fu_threads(n), sizeof(FusedSmem<n>), SBG_NP, st, J, tw_f, tw_i, sc, err);     \
         break;
         SBG_FUSED_CASES(SBG_LAUNCH_FU)
 #undef SBG_LAUNCH_FU
@@ -2033,6 +2033,20 @@ cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const L
     cudaError_t e = cudaSuccess;
     const bool pdl = alone && (int64_t)njobs * code_len(lgL) <= SBG_PDL_POINTS;
     KT_BEGIN(kt, KID_BATCH, st);
+    if (lgL >= SBG_FUSED_MIN_LG && lgL <= SBG_SMALL_MAX_LG) {
+        switch (lgL) {
+#define SBG_LAUNCH_FUB(n)                                                                                             \
+    case n:                                                                                                           \
+        e = launch_pdl(k_fused_b<n>, pdl, (int64_t)njobs * SBG_NP, fu_threads(n), sizeof(FusedSmem<n>), SBG_NP, st,    \
+                       djobs, tw_f, tw_i, sc, err);                                                                   \
+        break;
+            SBG_FUSED_CASES(SBG_LAUNCH_FUB)
+#undef SBG_LAUNCH_FUB
+            default: return cudaErrorInvalidValue;
+        }
+        KT_END(kt, KID_BATCH, st);
+        return e;
+    }
     if (lgL <= SBG_SMALL_MAX_LG) {
         size_t smem = (size_t)2 * padded_len(1 << lgL) * 4;
         e = launch_pdl(k_small_b, pdl, (int64_t)njobs * SBG_NP, 256, smem, 1, st, djobs, lgL, tw_f, tw_i, sc, flags,
