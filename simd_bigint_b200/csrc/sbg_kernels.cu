@@ -1952,8 +1952,17 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
         return cudaGetLastError();
     }
     const int64_t col_blocks = ((int64_t)col_ntiles(lgN1) * SBG_NP) << col_lgc(lgN1);
+    const bool coln = lgN1 <= COLN_MAX_LG && !split;
     KT_BEGIN(kt, KID_COL_FWD, st);
-    switch (lgN1) {
+    if (coln) switch (lgN1) {
+#define SBG_LAUNCH_FN(n)                                                                                          \
+    case n:                                                                                                       \
+        e = launch_pdl(k_coln_fwd<n>, pdl, (int64_t)nops * SBG_NP * COLN_TILES, COLN_T, 0, 1, st, a, an, b, bn,    \
+                       tw_f, YA, YB);                                                                             \
+        break;
+        SBG_COLN_CASES(SBG_LAUNCH_FN)
+#undef SBG_LAUNCH_FN
+    } else switch (lgN1) {
 #define SBG_LAUNCH_F(n)                                                                          \
     case n:                                                                                      \
         if (split) {                                                                             \
@@ -1978,7 +1987,12 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
     KT_END(kt, KID_ROW, st);
     if (e != cudaSuccess) return e;
     KT_BEGIN(kt, KID_COL_INV, st);
-    switch (lgN1) {
+    if (coln) switch (lgN1) {
+#define SBG_LAUNCH_IN(n)                                                                                          \
+    case n: e = launch_pdl(k_coln_inv<n>, pdl, (int64_t)SBG_NP * COLN_TILES, COLN_T, 0, 1, st, YA, tw_i); break;
+        SBG_COLN_CASES(SBG_LAUNCH_IN)
+#undef SBG_LAUNCH_IN
+    } else switch (lgN1) {
 #define SBG_LAUNCH_I(n) \
     case n: e = launch_col(k_col_inv<n>, pdl, n, col_blocks, st, YA, tw_i); break;
         SBG_COL_CASES(SBG_LAUNCH_I)
