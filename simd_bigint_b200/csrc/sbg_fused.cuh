@@ -369,8 +369,14 @@ struct RowlSmem {
     uint2 i[16];                               // their inverses times the CRT scale
 };
 
+// more than half an SM's shared memory: while the column kernel's CTAs are
+// still leaving, the scheduler would put two rows on one SM and none on another
+// (40 rows: 13 instead of 9 us)
+#define ROWL_SMEM (size_t)(120 << 10)
+static_assert(sizeof(RowlSmem) <= ROWL_SMEM, "row tables");
+
 template <bool BATCH>
-__global__ void __launch_bounds__(FU_T, 2) k_rowl(uint32_t* __restrict__ YA, const uint32_t* __restrict__ YB, int sq,
+__global__ void __launch_bounds__(FU_T, 1) k_rowl(uint32_t* __restrict__ YA, const uint32_t* __restrict__ YB, int sq,
                                                   const JobDesc* __restrict__ jobs, int lgN1, int m3, FsTables fsf,
                                                   FsTables fsi, ScaleArg sc, const uint2* __restrict__ twf,
                                                   const uint2* __restrict__ twi, uint32_t* flags, int64_t nflags) {
@@ -483,9 +489,9 @@ static cudaError_t fused_attr() {
     SBG_FUSED_CASES(SBG_FUSED_ATTR)
 #undef SBG_FUSED_ATTR
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_rowl<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowlSmem));
+        e = cudaFuncSetAttribute(k_rowl<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ROWL_SMEM);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_rowl<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowlSmem));
+        e = cudaFuncSetAttribute(k_rowl<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ROWL_SMEM);
     return e;
 }
 

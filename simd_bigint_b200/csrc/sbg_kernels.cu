@@ -1855,7 +1855,7 @@ static cudaError_t launch_rows(uint32_t* YA, const uint32_t* YB, int sq, const L
     const FsTables fsf{lp->fs_lo_f, lp->fs_hi_f, lp->hi_n}, fsi{lp->fs_lo_i, lp->fs_hi_i, lp->hi_n};
     const int64_t rows = SBG_NP * (lp->L >> ROW_LG);
     if (rows <= ROWL_MAX)
-        return launch_pdl(k_rowl<false>, pdl, rows, FU_T, sizeof(RowlSmem), 1, st, YA, YB, sq, (const JobDesc*)nullptr,
+        return launch_pdl(k_rowl<false>, pdl, rows, FU_T, ROWL_SMEM, 1, st, YA, YB, sq, (const JobDesc*)nullptr,
                           lp->lgN1, lp->m3, fsf, fsi, sc, tw_f, tw_i, flags, nflags);
     return launch_pdl(k_row12, pdl, rows, 256, 0, 1, st, YA, YB, sq, lp->lgN1, lp->m3, fsf, fsi, sc, tw_f, tw_i, flags,
                       nflags);
@@ -1866,7 +1866,7 @@ static cudaError_t launch_rows_b(const JobDesc* djobs, int njobs, const LenPlan*
     const FsTables fsf{lp->fs_lo_f, lp->fs_hi_f, lp->hi_n}, fsi{lp->fs_lo_i, lp->fs_hi_i, lp->hi_n};
     const int64_t rows = SBG_NP * (lp->L >> ROW_LG) * njobs;
     if (alone && rows <= ROWL_MAX)
-        return launch_pdl(k_rowl<true>, pdl, rows, FU_T, sizeof(RowlSmem), 1, st, (uint32_t*)nullptr,
+        return launch_pdl(k_rowl<true>, pdl, rows, FU_T, ROWL_SMEM, 1, st, (uint32_t*)nullptr,
                           (const uint32_t*)nullptr, 0, djobs, lp->lgN1, lp->m3, fsf, fsi, sc, tw_f, tw_i, flags, nflags);
     return launch_pdl(k_row12_b, pdl, rows, 256, 0, 1, st, djobs, lp->lgN1, lp->m3, fsf, fsi, sc, tw_f, tw_i, flags,
                       nflags);
