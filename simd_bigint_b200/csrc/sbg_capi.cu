@@ -44,14 +44,15 @@ int lg_ceil(int64_t n) {
 }
 
 // Transform length (code) for a convolution whose wanted coefficients need
-// L >= need: 2^a >= need, or 3 * 2^b >= need when that is shorter and bit b
-// of `mask3` allows it (the context's choice per size class, sbg_ctx_autotune).
+// L >= need: 2^a >= need, or 3 * 2^b >= need when that is shorter and b is
+// 12 .. 15, or bit b of `mask3` allows it (the context's choice per size
+// class, sbg_ctx_autotune).
 int conv_lg(int64_t need, uint32_t mask3) {
     int l = lg_ceil(need);
     if (l < 4) l = 4;
     int k = lg_ceil((need + 2) / 3);
-    if (k >= SBG_THREE_MIN_LG && k <= SBG_MAX_LG - 2 && ((int64_t)3 << k) < ((int64_t)1 << l) &&
-        ((mask3 >> k) & 1u))
+    if (k >= SBG_THREE_SHORT_LG && k <= SBG_MAX_LG - 2 && ((int64_t)3 << k) < ((int64_t)1 << l) &&
+        (k < SBG_THREE_MIN_LG || ((mask3 >> k) & 1u)))
         return SBG_CODE3 + k;
     return l;
 }
@@ -73,7 +74,7 @@ int ensure_plan(sbg_ctx* c, int lgL) {
         } else {
             np.lgN1 = lgL - 12;
         }
-        np.hi_n = (int)(np.L >> 13);
+        np.hi_n = (int)((np.L + 8191) >> 13);
         size_t lo_b = (size_t)SBG_NP * 8192 * sizeof(uint2);
         size_t hi_b = (size_t)SBG_NP * np.hi_n * sizeof(uint2);
         const size_t t3_b = np.m3 >= 0 ? (size_t)SBG_NP * (2 << np.m3) * sizeof(uint2) : 0;
@@ -720,7 +721,7 @@ int sbg_ctx_reserve(sbg_ctx* c, int64_t total) {
     CK(cudaSetDevice(c->device));
     int lg = conv_lg(total - 1, c->len3_mask);
     for (int l = 4; l <= SBG_NCODES; ++l) {            // every length up to the largest
-        if (l > SBG_MAX_LG && l < SBG_CODE3 + SBG_THREE_MIN_LG) continue;
+        if (l > SBG_MAX_LG && l < SBG_CODE3 + SBG_THREE_SHORT_LG) continue;
         if (code_len(l) > code_len(lg)) continue;
         int st = ensure_plan(c, l);
         if (st) return st;

@@ -346,6 +346,118 @@ __global__ void __launch_bounds__(COLN_T) k_coln_inv(uint32_t* __restrict__ YA, 
 }
 #define SBG_COLN_CASES(X) X(1) X(2) X(3) X(4)
 
+// ------------------------------------------------------------------------
+// Columns of 3 * 2^m rows, m = 0 .. 3 (transforms of 3 * 2^12 .. 3 * 2^15
+// points): a thread per column holds all its rows; the radix-3 level over the
+// thirds, then a 2^m-point DIF per third, as in the longer 3 * 2^m columns.
+// CPT columns per thread: one for a lone product, more for a batch's jobs.
+// ------------------------------------------------------------------------
+#define COL3N_MAX 3
+__host__ __device__ constexpr int col3n_cpt(int m) { return m <= 1 ? 4 : (m == 2 ? 2 : 1); }
+__host__ __device__ constexpr int col3n_tiles(int cpt) { return COLN_TILES / cpt; }
+template <int M3, int CPT>
+__device__ __forceinline__ void col3n_fwd_body(int q, int tile, const uint64_t* __restrict__ X, int64_t xn,
+                                               const uint2* __restrict__ twf, const Radix3Arg& r3,
+                                               uint32_t* __restrict__ Y) {
+    constexpr int M = 1 << M3;
+    const PrimeConst pc = c_pr[q];
+    const uint2* tw = twf + (size_t)q * SBG_TW_N;
+    const uint2* t3 = r3.t3 + ((size_t)q << (M3 + 1));
+    Y += (size_t)q * (3 * M) << SBG_ROW_LG;
+#pragma unroll 1
+    for (int i = 0; i < CPT; ++i) {
+        const int c = (tile * CPT + i) * COLN_T + threadIdx.x;
+        uint32_t x[M], y[M], z[M];
+#pragma unroll
+        for (int r = 0; r < M; ++r) {
+            x[r] = load_limb(X, xn, ((int64_t)r << SBG_ROW_LG) + c, pc);
+            y[r] = load_limb(X, xn, ((int64_t)(r + M) << SBG_ROW_LG) + c, pc);
+            z[r] = load_limb(X, xn, ((int64_t)(r + 2 * M) << SBG_ROW_LG) + c, pc);
+        }
+#pragma unroll
+        for (int r = 0; r < M; ++r)
+            r3_dif(x[r], y[r], z[r], r3.w[q], r3.ws[q], __ldg(&t3[r]), __ldg(&t3[2 * r]), pc.p);
+        if constexpr (M > 1) {
+            dif_regs2<M, true>(x, y, tw, 0, 1, M3, pc.p);
+            dif_regs<M, true>(z, tw, 0, 1, M3, pc.p);
+        }
+        uint32_t* out = Y + c;
+#pragma unroll
+        for (int r = 0; r < M; ++r) {
+            out[r << SBG_ROW_LG] = x[r];
+            out[(r + M) << SBG_ROW_LG] = y[r];
+            out[(r + 2 * M) << SBG_ROW_LG] = z[r];
+        }
+    }
+}
+template <int M3, int CPT>
+__device__ __forceinline__ void col3n_inv_body(int q, int tile, uint32_t* __restrict__ Y, const uint2* __restrict__ twi,
+                                               const Radix3Arg& r3) {
+    constexpr int M = 1 << M3;
+    const PrimeConst pc = c_pr[q];
+    const uint2* tw = twi + (size_t)q * SBG_TW_N;
+    const uint2* t3 = r3.t3 + ((size_t)q << (M3 + 1));
+    Y += (size_t)q * (3 * M) << SBG_ROW_LG;
+#pragma unroll 1
+    for (int i = 0; i < CPT; ++i) {
+        uint32_t* col = Y + (tile * CPT + i) * COLN_T + threadIdx.x;
+        uint32_t x[M], y[M], z[M];
+#pragma unroll
+        for (int r = 0; r < M; ++r) {
+            x[r] = __ldcg(&col[r << SBG_ROW_LG]);
+            y[r] = __ldcg(&col[(r + M) << SBG_ROW_LG]);
+            z[r] = __ldcg(&col[(r + 2 * M) << SBG_ROW_LG]);
+        }
+        if constexpr (M > 1) {
+            dit_regs2<M, true>(x, y, tw, 0, 1, M3, pc.p);
+            dit_regs<M, true>(z, tw, 0, 1, M3, pc.p);
+        }
+#pragma unroll
+        for (int r = 0; r < M; ++r) {
+            r3_dit(x[r], y[r], z[r], r3.w[q], r3.ws[q], __ldg(&t3[r]), __ldg(&t3[2 * r]), pc.p);
+            col[r << SBG_ROW_LG] = x[r];
+            col[(r + M) << SBG_ROW_LG] = y[r];
+            col[(r + 2 * M) << SBG_ROW_LG] = z[r];
+        }
+    }
+}
+template <int M3>
+__global__ void __launch_bounds__(COLN_T) k_col3n_fwd(const uint64_t* __restrict__ a, int64_t an,
+                                                      const uint64_t* __restrict__ b, int64_t bn,
+                                                      const uint2* __restrict__ twf, Radix3Arg r3,
+                                                      uint32_t* __restrict__ YA, uint32_t* __restrict__ YB) {
+    pdl_enter();
+    const int tile = blockIdx.x % COLN_TILES, q = blockIdx.x / COLN_TILES % SBG_NP, op = blockIdx.x / (COLN_TILES * SBG_NP);
+    col3n_fwd_body<M3, 1>(q, tile, op ? b : a, op ? bn : an, twf, r3, op ? YB : YA);
+}
+template <int M3>
+__global__ void __launch_bounds__(COLN_T) k_col3n_inv(uint32_t* __restrict__ YA, const uint2* __restrict__ twi,
+                                                      Radix3Arg r3) {
+    pdl_enter();
+    col3n_inv_body<M3, 1>(blockIdx.x / COLN_TILES, blockIdx.x % COLN_TILES, YA, twi, r3);
+}
+// batched: blocks (job, operand, prime, tile), job slowest
+template <int M3>
+__global__ void __launch_bounds__(COLN_T) k_col3n_fwd_b(const JobDesc* __restrict__ jobs, const uint2* __restrict__ twf,
+                                                        Radix3Arg r3) {
+    pdl_enter();
+    constexpr int CPT = col3n_cpt(M3), NT = col3n_tiles(CPT), PER_JOB = 2 * SBG_NP * NT;
+    const JobDesc& J = jobs[blockIdx.x / PER_JOB];
+    const int r = blockIdx.x % PER_JOB, op = r / (SBG_NP * NT);
+    if (op && J.sq) return;
+    uint32_t* Y = J.ws + (op ? (size_t)SBG_NP * (3 << M3) << SBG_ROW_LG : 0);
+    col3n_fwd_body<M3, CPT>(r / NT % SBG_NP, r % NT, op ? J.b : J.a, op ? J.bn : J.an, twf, r3, Y);
+}
+template <int M3>
+__global__ void __launch_bounds__(COLN_T) k_col3n_inv_b(const JobDesc* __restrict__ jobs, const uint2* __restrict__ twi,
+                                                        Radix3Arg r3) {
+    pdl_enter();
+    constexpr int CPT = col3n_cpt(M3), NT = col3n_tiles(CPT), PER_JOB = SBG_NP * NT;
+    const int r = blockIdx.x % PER_JOB;
+    col3n_inv_body<M3, CPT>(r / NT, r % NT, jobs[blockIdx.x / PER_JOB].ws, twi, r3);
+}
+#define SBG_COL3N_CASES(X) X(0) X(1) X(2) X(3)
+
 #define SBG_FUSED_CASES(X) X(8) X(9) X(10) X(11) X(12)
 
 // ------------------------------------------------------------------------

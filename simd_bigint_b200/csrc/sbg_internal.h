@@ -66,11 +66,14 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), bool pdl, int64_t blocks, 
 #endif
 
 // Transform lengths are identified by a code: c <= SBG_MAX_LG is L = 2^c,
-// c = SBG_CODE3 + k is L = 3 * 2^k (four-step only, k >= SBG_THREE_MIN_LG),
+// c = SBG_CODE3 + k is L = 3 * 2^k (four-step only, k >= SBG_THREE_SHORT_LG),
 // chosen when it is the smaller of the two lengths that hold a product.
 #define SBG_CODE3 32
 #define SBG_NCODES (SBG_CODE3 + SBG_MAX_LG)
 #define SBG_THREE_MIN_LG 16
+// k = 12 .. 15 are always used: their columns have at most 24 rows, so the
+// radix-3 level needs no exchange and the quarter of the points saved is saved
+#define SBG_THREE_SHORT_LG 12
 // k = 16..19 and 21..23: where 3 * 2^k measured faster than 2^(k+2) on B200
 // (at k = 20 the columns of 768 rows need the cross-CTA radix-3 exchange,
 // which costs more than the quarter of the points it saves)
@@ -111,7 +114,7 @@ struct LenPlan {
     uint32_t w3f[SBG_NP] = {}, w3fs[SBG_NP] = {};   // cube roots of unity (forward)
     uint32_t w3i[SBG_NP] = {}, w3is[SBG_NP] = {};   // and their inverses
     uint2* fs_lo_f = nullptr;     // [q][8192]      w_L^e, e < 2^13
-    uint2* fs_hi_f = nullptr;     // [q][L >> 13]   w_L^(e << 13)
+    uint2* fs_hi_f = nullptr;     // [q][ceil(L / 2^13)]   w_L^(e << 13)
     uint2* fs_lo_i = nullptr;
     uint2* fs_hi_i = nullptr;
     int hi_n = 0;                 // entries in each hi table

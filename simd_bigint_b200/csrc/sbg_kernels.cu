@@ -1914,6 +1914,13 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
         break;
             SBG_COL3S_CASES(SBG_LAUNCH_F3S)
 #undef SBG_LAUNCH_F3S
+#define SBG_LAUNCH_F3N(n)                                                                                        \
+    case n:                                                                                                      \
+        e = launch_pdl(k_col3n_fwd<n>, pdl, (int64_t)nops * SBG_NP * COLN_TILES, COLN_T, 0, 1, st, a, an, b, bn,  \
+                       tw_f, r3f, YA, YB);                                                                       \
+        break;
+            SBG_COL3N_CASES(SBG_LAUNCH_F3N)
+#undef SBG_LAUNCH_F3N
 #define SBG_LAUNCH_F3(n)                                                                          \
     case n:                                                                                       \
         e = launch_colx(k_col3_fwd<n>, pdl, (int64_t)nops * col3_ntiles(n) * SBG_NP * col3_csize(n),    \
@@ -1938,6 +1945,12 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
         break;
             SBG_COL3S_CASES(SBG_LAUNCH_I3S)
 #undef SBG_LAUNCH_I3S
+#define SBG_LAUNCH_I3N(n)                                                                                         \
+    case n:                                                                                                       \
+        e = launch_pdl(k_col3n_inv<n>, pdl, (int64_t)SBG_NP * COLN_TILES, COLN_T, 0, 1, st, YA, tw_i, r3i);        \
+        break;
+            SBG_COL3N_CASES(SBG_LAUNCH_I3N)
+#undef SBG_LAUNCH_I3N
 #define SBG_LAUNCH_I3(n)                                                                             \
     case n:                                                                                          \
         e = launch_colx(k_col3_inv<n>, pdl, (int64_t)col3_ntiles(n) * SBG_NP * col3_csize(n),               \
@@ -2077,6 +2090,13 @@ cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const L
         break;
             SBG_COL3S_CASES(SBG_LAUNCH_FB3S)
 #undef SBG_LAUNCH_FB3S
+#define SBG_LAUNCH_FB3N(n)                                                                                       \
+    case n:                                                                                                      \
+        e = launch_pdl(k_col3n_fwd_b<n>, pdl, (int64_t)njobs * 2 * SBG_NP * col3n_tiles(col3n_cpt(n)), COLN_T, 0, \
+                       1, st, djobs, tw_f, r3f);                                                                 \
+        break;
+            SBG_COL3N_CASES(SBG_LAUNCH_FB3N)
+#undef SBG_LAUNCH_FB3N
 #define SBG_LAUNCH_FB3(n)                                                                       \
     case n:                                                                                     \
         e = launch_colx(k_col3_fwd_b<n>, pdl, (int64_t)njobs * 2 * col3_ntiles(n) * SBG_NP * col3_csize(n), \
@@ -2097,6 +2117,13 @@ cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const L
         break;
             SBG_COL3S_CASES(SBG_LAUNCH_IB3S)
 #undef SBG_LAUNCH_IB3S
+#define SBG_LAUNCH_IB3N(n)                                                                                    \
+    case n:                                                                                                   \
+        e = launch_pdl(k_col3n_inv_b<n>, pdl, (int64_t)njobs * SBG_NP * col3n_tiles(col3n_cpt(n)), COLN_T, 0, \
+                       1, st, djobs, tw_i, r3i);                                                              \
+        break;
+            SBG_COL3N_CASES(SBG_LAUNCH_IB3N)
+#undef SBG_LAUNCH_IB3N
 #define SBG_LAUNCH_IB3(n)                                                                     \
     case n:                                                                                   \
         e = launch_colx(k_col3_inv_b<n>, pdl, (int64_t)njobs * col3_ntiles(n) * SBG_NP * col3_csize(n), \

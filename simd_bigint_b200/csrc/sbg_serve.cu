@@ -409,7 +409,7 @@ extern "C" int sbg_server_create(sbg_ctx* ctx, const sbg_server_config* cfg, sbg
     do {
         if ((st = cuda_fail(cudaSetDevice(ctx->device), "device"))) break;
         for (int l = 4; l <= 22 && !st; ++l) st = ensure_plan(ctx, l);   // tables to 2^22 points
-        for (int k = SBG_THREE_MIN_LG; k <= 20 && !st; ++k) st = ensure_plan(ctx, SBG_CODE3 + k);
+        for (int k = SBG_THREE_SHORT_LG; k <= 20 && !st; ++k) st = ensure_plan(ctx, SBG_CODE3 + k);
         if (st) break;
         // stream priorities: multiply slots highest, reciprocal workers lowest,
         // so short multiplies are not queued behind long Newton batches
