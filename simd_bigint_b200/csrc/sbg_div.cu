@@ -280,6 +280,39 @@ __device__ uint32_t block_fold3(Grp<CL>& grp, uint64_t* P, int64_t L, const uint
     return ca | (cb << 1) | (cc << 2);
 }
 
+// z[0..len) = x - y + w in one pass over the tiles, carries out of the top dropped
+template <int CL, class FX, class FY, class FW>
+__device__ void block_sub_add(Grp<CL>& grp, uint64_t* z, int64_t len, FX x, FY y, FW w) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    constexpr int64_t TILE = (int64_t)DIV_T * FOLD_PER;
+    uint32_t cb = 0, cc = 0;
+    for (int64_t base = 0; base < len; base += (int64_t)CL * TILE) {
+        const int64_t w0 = base + (int64_t)grp.rank * TILE + (int64_t)wid * (32 * FOLD_PER) + lane;
+        uint64_t v[FOLD_PER], nh[FOLD_PER];
+        uint32_t g[FOLD_PER], p[FOLD_PER], cm[FOLD_PER];
+#pragma unroll
+        for (int k = 0; k < FOLD_PER; ++k) {
+            const int64_t i = w0 + 32 * k;
+            const bool in = i < len;
+            nh[k] = in ? w(i) : 0;
+            chain_row(in ? x(i) : 0, in ? y(i) : 0, in, true, v[k], g[k], p[k]);
+        }
+        cb = tile_carries(grp, g, p, cb, cm);
+#pragma unroll
+        for (int k = 0; k < FOLD_PER; ++k) {
+            const int64_t i = w0 + 32 * k;
+            const bool in = i < len;
+            chain_row(in ? v[k] - ((cm[k] >> lane) & 1u) : 0, nh[k], in, false, v[k], g[k], p[k]);
+        }
+        cc = tile_carries(grp, g, p, cc, cm);
+#pragma unroll
+        for (int k = 0; k < FOLD_PER; ++k) {
+            const int64_t i = w0 + 32 * k;
+            if (i < len) z[i] = v[k] + ((cm[k] >> lane) & 1u);
+        }
+    }
+}
+
 // sign of x - y over len limbs: -1, 0, 1 (group-uniform).  Walks down from
 // the top CL * DIV_T limbs at a time and stops at the first window holding a
 // difference (the top one, unless the operands agree there).
@@ -726,6 +759,29 @@ __device__ void recip_step1(Grp<CL>& grp, const RecipStep& S, uint32_t* err) {
                  [&](int64_t i) { return 0ull; }, false, cin);
 }
 
+// The least k in 1 .. kmax with k A > E for an (n+1)-limb E = (e2, e1, e0, ..)
+// and a normalised n-limb A = (a1, a0, ..), by those limbs (k A lies between
+// its two-limb top and that plus k); 0 where they do not settle it.
+__device__ __forceinline__ int least_multiple(uint64_t e2, uint64_t e1, uint64_t e0, uint64_t a1, uint64_t a0, int kmax) {
+    const unsigned __int128 e = ((unsigned __int128)e1 << 64) | e0, a = ((unsigned __int128)a1 << 64) | a0;
+    unsigned __int128 ka = 0;
+    uint64_t ka2 = 0;
+    for (int q = 1; q <= kmax; ++q) {
+        ka += a;
+        ka2 += ka < a;
+        if (e2 < ka2 || (e2 == ka2 && e < ka)) return q;
+        const unsigned __int128 kb = ka + q;                // at most k above
+        const uint64_t kb2 = ka2 + (kb < ka);
+        if (e2 < kb2 || (e2 == kb2 && e < kb)) return 0;
+    }
+    return 0;
+}
+
+// limb i of the n-limb A times 2^b, b >= 1
+__device__ __forceinline__ uint64_t limb_shl(const uint64_t* A, int64_t n, int64_t i, int b) {
+    return (i < n ? A[i] << b : 0ull) | (i > 0 ? A[i - 1] >> (64 - b) : 0ull);
+}
+
 // Steps 0 and 1 in one kernel.  Nearly always a handful of limbs, which every
 // thread reads, settles what the general code above finds with passes and
 // barriers over the whole number:
@@ -795,33 +851,13 @@ __global__ void __launch_bounds__(DIV_T) k_recip_mid(const RecipStep* st, uint32
     int k = 0;
     const uint64_t x0 = S.Xh[0];
     if (fast) {
-        // the least k with k A > E, by the top limbs: k A lies between its
-        // two-limb top and that plus k
-        const unsigned __int128 e = ((unsigned __int128)E(n - 1) << 64) | E(n - 2);
-        const unsigned __int128 a = ((unsigned __int128)A[n - 1] << 64) | A[n - 2];
-        const uint64_t e2 = E(n);
-        unsigned __int128 ka = 0;
-        uint64_t ka2 = 0;
-        for (int q = 1; q <= 4 && !k; ++q) {
-            ka += a;
-            ka2 += ka < a;
-            if (e2 < ka2 || (e2 == ka2 && e < ka)) {
-                k = q;
-            } else {
-                const unsigned __int128 kb = ka + q;        // at most k above
-                const uint64_t kb2 = ka2 + (kb < ka);
-                if (e2 < kb2 || (e2 == kb2 && e < kb)) break;
-            }
-        }
+        k = least_multiple(E(n), E(n - 1), E(n - 2), A[n - 1], A[n - 2], 4);
     }
     if (k) {
         auto put = [&](int64_t i, uint64_t v) {
             if (i >= l) TM[i - l] = v;
         };
-        // limb i of A 2^b, b >= 1
-        auto shl = [&](int64_t i, int b) -> uint64_t {
-            return (i < n ? A[i] << b : 0ull) | (i > 0 ? A[i - 1] >> (64 - b) : 0ull);
-        };
+        auto shl = [&](int64_t i, int b) { return limb_shl(A, n, i, b); };
         uint32_t bor;
         if (k == 1) {
             bor = block_store(grp, put, n + 1, [&](int64_t i) { return i < n ? A[i] : 0ull; }, E, true, 0);
@@ -916,7 +952,36 @@ __global__ void __launch_bounds__(DIV_T) k_div_fix(const DivFix* df, uint32_t* e
     uint64_t* P = F.P;
     const uint64_t* D = F.D;
     uint64_t* Rw = F.Rw;
-    if (F.L == 0) {
+    // With S = N_lo + N_hi - C_lo - C_hi = R + d (B^L - 1): limb L-1 of R - d is
+    // zero or all ones, so d is the top limbs' sum rounded to a multiple of B, and
+    // R is S + d on its n+1 limbs: d and the three limbs of C_hi go into the lowest
+    // four of C, and N - C' + N_hi is one pass.  Where limb 3 does not end the
+    // carry, the general fold over L limbs runs.
+    bool settled = false;
+    uint64_t f0 = 0, f1 = 0, f2 = 0, f3 = 0;
+    if (F.L > 0 && n >= 4) {
+        const int64_t L = F.L;
+        const __int128 top = (__int128)N[L - 1] + (2 * L - 1 < 2 * n ? N[2 * L - 1] : 0) - P[L - 1];
+        const __int128 d = (top + ((__int128)1 << 63)) >> 64;
+        const __int128 off = top - (d << 64);
+        settled = off >= -4 && off <= 4 && d >= -2 && d <= 2;
+        const uint64_t g0 = P[L], g1 = P[L + 1], g2 = P[L + 2];
+        __int128 t = (__int128)P[0] + g0 - d;
+        f0 = (uint64_t)t;
+        t = (__int128)P[1] + g1 + (t >> 64);
+        f1 = (uint64_t)t;
+        t = (__int128)P[2] + g2 + (t >> 64);
+        f2 = (uint64_t)t;
+        t = (__int128)P[3] + (t >> 64);
+        f3 = (uint64_t)t;
+        settled = settled && (t >> 64) == 0;
+    }
+    if (settled) {
+        const int64_t L = F.L;
+        block_sub_add(grp, Rw, n + 1, [&](int64_t i) { return N[i]; },
+                      [&](int64_t i) { return i < 4 ? (i == 0 ? f0 : (i == 1 ? f1 : (i == 2 ? f2 : f3))) : P[i]; },
+                      [&](int64_t i) { return L + i < 2 * n ? N[L + i] : 0ull; });
+    } else if (F.L == 0) {
         block_addsub(grp, Rw, n + 1, [&](int64_t i) { return N[i]; }, [&](int64_t i) { return P[i]; },
                      true, 0);
     } else {
@@ -957,6 +1022,40 @@ __global__ void __launch_bounds__(DIV_T) k_div_fix(const DivFix* df, uint32_t* e
         } else {
             GRP_LOOP(i, n + 1) Rw[i] = P[i];
         }
+    }
+    grp.sync();
+    // how many times D still goes into R (at most five)
+    const int k = n >= 4 ? least_multiple(Rw[n], Rw[n - 1], Rw[n - 2], D[n - 1], D[n - 2], 6) : 0;
+    if (k > 0) {
+        const uint64_t q0 = F.Q[0];
+        uint64_t* R = F.R;
+        auto put = [&](int64_t i, uint64_t v) {
+            if (i < n) R[i] = v;
+        };
+        auto rw = [&](int64_t i) { return Rw[i]; };
+        int m = k - 1;                          // 0, 1, 2, 4, or 3 and 5 in two passes
+        if (m == 3 || m == 5) {
+            block_addsub(grp, Rw, n + 1, rw, [&](int64_t i) { return i < n ? D[i] : 0ull; }, true, 0);
+            --m;
+        }
+        if (m == 0) {
+            GRP_LOOP(i, n) R[i] = Rw[i];
+        } else if (m == 1) {
+            block_store(grp, put, n + 1, rw, [&](int64_t i) { return i < n ? D[i] : 0ull; }, true, 0);
+        } else {
+            block_store(grp, put, n + 1, rw, [&](int64_t i) { return limb_shl(D, n, i, m >> 1); }, true, 0);
+        }
+        m = k - 1;
+        if (q0 + (uint64_t)m >= q0) {           // read by every thread before a barrier when m > 0
+            if (m && grp.rank == 0 && threadIdx.x == 0) F.Q[0] = q0 + m;
+        } else {
+            for (int j = 0; j < m; ++j) {
+                block_step1(grp, F.Q, n + 1, true);
+                grp.sync();
+            }
+        }
+        if constexpr (CL > 1) grp.sync();
+        return;
     }
     for (int it = 0; it < 8; ++it) {
         grp.sync();
