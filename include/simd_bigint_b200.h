@@ -77,13 +77,14 @@ int sbg_ctx_set_timing(sbg_ctx *ctx, int on);
 /* Number of kernel launches this context has queued so far (diagnostics). */
 int64_t sbg_ctx_launches(sbg_ctx *ctx);
 /* Transform lengths.  A product of N coefficients runs at L = 2^a >= N or,
- * for 2^(k+1) < N <= 3 * 2^k with 16 <= k <= 23, at L = 3 * 2^k when bit k
- * of the context's mask is set.  sbg_ctx_autotune times one product of each
- * such size class at both lengths on this device (about a second; allocates
- * 400 MB temporarily) and sets the mask to the faster; times (optional, 16
- * doubles) receives {ms at 2^(k+2), ms at 3 * 2^k} for k = 16 .. 23.  No
- * counterpart in the reference (its p30 engine picks lengths by its own
- * table, include/p30.h:31-37). */
+ * for 2^(k+1) < N <= 3 * 2^k, at L = 3 * 2^k: always for 12 <= k <= 15, and
+ * for 16 <= k <= 23 when bit k of the context's mask is set.
+ * sbg_ctx_autotune times one product of each of those eight size classes at
+ * both lengths on this device (about a second; allocates 400 MB temporarily)
+ * and sets the mask to the faster; times (optional, 16 doubles) receives
+ * {ms at 2^(k+2), ms at 3 * 2^k} for k = 16 .. 23.  No counterpart in the
+ * reference (its p30 engine picks lengths by its own table,
+ * include/p30.h:31-37). */
 int sbg_ctx_autotune(sbg_ctx *ctx, double *times);
 int sbg_ctx_set_len3_mask(sbg_ctx *ctx, uint32_t mask);
 uint32_t sbg_ctx_get_len3_mask(sbg_ctx *ctx);
@@ -338,7 +339,9 @@ int sbg_noalloc_status(void *stream);
  *   SBG_INJECT_WITHHOLD  the first block of each carry scan never publishes
  *                        its look-back flag, and the look-back's bounded wait
  *                        is shortened, so the next block's wait runs out:
- *                        the product is wrong and the status SBG_ETIMEOUT;
+ *                        the product is wrong and the status SBG_ETIMEOUT
+ *                        (products of 2^8 .. 2^12 transform points resolve
+ *                        their carries without a flag and are not affected);
  *   SBG_INJECT_TOP       the top coefficient's first residue is altered
  *                        before Garner: the product spills, SBG_ESPILL;
  *   SBG_INJECT_MID       a middle coefficient's residue is altered: a wrong

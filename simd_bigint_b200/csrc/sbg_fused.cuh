@@ -467,9 +467,8 @@ __global__ void __launch_bounds__(COLN_T) k_col3n_inv_b(const JobDesc* __restric
 // spent waiting for twiddles that no other CTA has brought to L1.  Here a row
 // has 512 threads, an operand to each half, and its twiddles staged in shared
 // memory -- before the previous kernel of the chain is waited for, as the
-// tables are older than that.  Device time a launch: 14.5 -> 9.9 us for 10 to
-// 80 rows; with two such CTAs on an SM (160 rows: 17.3 us) k_row12
-// higher throughput wins (320 rows: both 17 us).
+// tables are older than that.  Device time a launch, 10 to 80 rows: 14.5 -> 9.9 us.
+// Beyond one row per SM k_row12 wins (160 rows: 17.3 us here, 15 to 17 there).
 // ------------------------------------------------------------------------
 #define ROWL_MAX 148
 struct RowlSmem {

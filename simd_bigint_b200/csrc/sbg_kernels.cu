@@ -10,7 +10,9 @@
 // 3 * 2^m): K1 / K3 transform its columns (tiles of adjacent columns, split
 // over thread-block clusters when a column is long; k_col3* for 3 * 2^m
 // rows), K2 its rows.  Transforms of L <= 2^12 points skip the four-step
-// split and run whole in one CTA per prime (k_small).  This is the reference's p30 pipeline
+// split: whole products in one cluster launch (k_fused), below 2^8 points and
+// for the allocation-free multiply one CTA per prime and a carry scan
+// (k_small).  This is the reference's p30 pipeline
 // (include/p30.h:1847-1938: input -> forward -> fused pointwise+inverse ->
 // scale -> Garner/carry), laid out as a four-step NTT over HBM: every pass
 // reads and writes each spectrum once, all levels inside a pass stay on chip.

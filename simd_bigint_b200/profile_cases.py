@@ -6,7 +6,7 @@ command, for capturing them under a profiler:
 Cases (operands seeded, resident on cuda:0, each call repeated `repeats`
 times, 3 by default, so a capture can skip the first launch):
 
-    small     one 1500 x 1500-limb product (single-CTA transforms, k_small,
+    small     one 1500 x 1500-limb product (one launch, k_fused;
               the short-product carry scan k_crt_carry_s)
     mid       one 16384 x 16384-limb product (four-step kernels at 2^15
               points, k_crt_carry_s)
