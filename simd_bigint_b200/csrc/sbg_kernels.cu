@@ -1879,7 +1879,7 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
                         uint32_t* ws, uint32_t* flags, int64_t nflags, cudaStream_t st, KTimer* kt,
                         cudaEvent_t b_ready) {
     const size_t L = (size_t)code_len(lgL);
-    const bool pdl = (int64_t)L <= SBG_PDL_POINTS;
+    const bool pdl = (int64_t)L <= SBG_PDL_POINTS && !b_ready;   // an event between two kernels keeps them whole
     // the first operand's forward columns may start before the second
     // operand has arrived only on the power-of-two four-step path
     const bool split = b_ready && !sq && lgL > SBG_SMALL_MAX_LG && lp->m3 < 0;
