@@ -1329,7 +1329,8 @@ static int div_core(sbg_ctx* c, std::vector<DivInst>& v, uint32_t* err, bool quo
         if ((rc = launch_lin(c, k_div_fix<1>, k_div_fix<DIV_CL>, (const DivFix*)dfx, fs, fb, err))) return rc;
         std::vector<CopyDesc> cq;
         cq.reserve(v.size());
-        for (auto& d : v) cq.push_back(CopyDesc{d.Q, d.Qout, d.qlen, d.qlen});
+        for (auto& d : v)
+            if (d.Q != d.Qout) cq.push_back(CopyDesc{d.Q, d.Qout, d.qlen, d.qlen});
         if ((rc = copy_batch(c, cq))) return rc;
     }
     return SBG_OK;
@@ -1408,6 +1409,30 @@ extern "C" int sbg_recip(sbg_ctx* c, uint64_t* ip, const uint64_t* dp, int64_t n
     return sbg::recip_batch(c, &dp, &ip, &n, 1);
 }
 
+// whether no output of the batch overlaps any other range of it
+static bool outputs_apart(const sbg_div_job* jobs, int64_t count) {
+    struct Range {
+        const uint64_t *lo, *hi;
+        bool out;
+    };
+    std::vector<Range> r;
+    r.reserve((size_t)count * 4);
+    for (int64_t i = 0; i < count; ++i) {
+        const sbg_div_job& j = jobs[i];
+        r.push_back({j.qp, j.qp + (j.nn - j.dn + 1), true});
+        r.push_back({j.rp, j.rp + j.dn, true});
+        r.push_back({j.np, j.np + j.nn, false});
+        r.push_back({j.dp, j.dp + j.dn, false});
+    }
+    std::sort(r.begin(), r.end(), [](const Range& a, const Range& b) { return a.lo < b.lo; });
+    const uint64_t *in_end = nullptr, *out_end = nullptr;      // furthest ends so far
+    for (const Range& x : r) {
+        if (x.lo < out_end || (x.out && x.lo < in_end)) return false;
+        (x.out ? out_end : in_end) = std::max(x.out ? out_end : in_end, x.hi);
+    }
+    return true;
+}
+
 // Batched division: every job has a normalised divisor (top bit set) and
 // nn <= 2 dn (the configurations of the reference's Newton division); other
 // shapes go through sbg_divrem, which normalises and splits them.  Queues the
@@ -1450,6 +1475,12 @@ static int divrem_enqueue(sbg_ctx* c, const sbg_div_job* jobs, int64_t count, bo
     v.reserve((size_t)count);
     cn.reserve((size_t)count);
     uint64_t* p = scratch;
+    // A full 2n-limb numerator is read, and its (n+1)-limb quotient built, where
+    // they are, unless an output of the batch overlaps another range: 128
+    // divisions of mixed sizes, 4942 -> 4818 us without the copies.
+    // Shorter numerators need the zero limbs above them, shorter quotients room
+    // for a top limb that is zero only after the correction.
+    const bool apart = outputs_apart(jobs, count);
     for (int64_t i = 0; i < count; ++i) {
         const sbg_div_job& j = jobs[i];
         if (j.dn <= SBG_DIV_BASE) continue;
@@ -1461,6 +1492,13 @@ static int divrem_enqueue(sbg_ctx* c, const sbg_div_job* jobs, int64_t count, bo
         d.Qout = j.qp;
         d.Rout = j.rp;
         d.qlen = j.nn - j.dn + 1;
+        if (apart && j.nn == 2 * j.dn) {
+            cn.pop_back();
+            d.N = j.np;
+            carve(d, p);
+            d.Q = j.qp;
+            continue;
+        }
         // numerator zero-padded to 2n limbs (one batched copy below)
         uint64_t* Np = p;
         p += 2 * j.dn + 8;

@@ -73,3 +73,33 @@ def test_structured_divisions(ctx, n):
         wq, wr = divmod(x, d)
         assert _int(q.cpu().numpy().view(np.uint64)) == wq, name
         assert _int(r.cpu().numpy().view(np.uint64)) == wr, name
+
+
+@pytest.mark.parametrize("n", [200, 3000, 8000])
+def test_results_over_the_numerator(ctx, n):
+    """Quotient or remainder written over the numerator, one division's over
+    another's, or all apart: the same results."""
+    import torch
+    rng = np.random.default_rng(n + 7)
+    for layout in ("apart", "remainder over own", "quotient over own", "over the other's"):
+        nums = [rng.integers(0, 2**64, 2 * n, dtype=np.uint64) for _ in range(2)]
+        divs = [rng.integers(0, 2**64, n, dtype=np.uint64) for _ in range(2)]
+        for d in divs:
+            d[-1] |= np.uint64(1 << 63)
+        tn, td = [_dev(x) for x in nums], [_dev(x) for x in divs]
+        q = [torch.empty(n + 1, dtype=torch.int64, device="cuda") for _ in range(2)]
+        r = [torch.empty(n, dtype=torch.int64, device="cuda") for _ in range(2)]
+        for i in range(2):
+            if layout == "remainder over own":
+                r[i] = tn[i][:n]
+            elif layout == "quotient over own":
+                q[i] = tn[i][: n + 1]
+            elif layout == "over the other's":
+                r[i] = tn[1 - i][n:]
+        torch.cuda.synchronize()
+        ctx.divrem_batch([(q[i].data_ptr(), r[i].data_ptr(), tn[i].data_ptr(), td[i].data_ptr(), 2 * n, n)
+                          for i in range(2)])
+        for i in range(2):
+            wq, wr = divmod(_int(nums[i]), _int(divs[i]))
+            assert _int(q[i].cpu().numpy().view(np.uint64)) == wq, layout
+            assert _int(r[i].cpu().numpy().view(np.uint64)) == wr, layout
