@@ -347,10 +347,14 @@ int sbg_noalloc_status(void *stream);
  *   SBG_INJECT_MID       a middle coefficient's residue is altered: a wrong
  *                        product that no device check sees (for host checks).
  * sbg_debug_fail_allocs(n): the next n device allocations of contexts
- * (workspace, plan tables) fail as an out-of-memory device would (SBG_EALLOC). */
+ * (workspace, plan tables) fail as an out-of-memory device would (SBG_EALLOC).
+ * sbg_debug_ring_bytes(n): descriptor rings allocated from now on hold n bytes,
+ * or four of the blocks that did not fit if that is more, so that short lists
+ * wrap them as very long ones would (0: their own sizes). */
 enum { SBG_INJECT_WITHHOLD = 1, SBG_INJECT_TOP = 2, SBG_INJECT_MID = 4 };
 int sbg_debug_inject(uint32_t mask);
 void sbg_debug_fail_allocs(int n);
+void sbg_debug_ring_bytes(int64_t n);
 
 /* ---- diagnostics ---------------------------------------------------------- */
 

@@ -129,6 +129,8 @@ def lib(build_if_missing: bool = False):
         L.sbg_debug_inject.restype = C.c_int
         L.sbg_debug_fail_allocs.argtypes = [C.c_int]
         L.sbg_debug_fail_allocs.restype = None
+        L.sbg_debug_ring_bytes.argtypes = [_i64]
+        L.sbg_debug_ring_bytes.restype = None
         L.sbg_noalloc_status.argtypes = [_vp]
         L.sbg_noalloc_status.restype = C.c_int
         L.sbg_mul_noalloc.argtypes = [_vp, _vp, _i64, _vp, _i64, _vp]

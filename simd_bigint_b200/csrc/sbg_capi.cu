@@ -29,6 +29,7 @@ int cuda_fail(cudaError_t e, const char* where) {
     } while (0)
 
 static std::atomic<int> g_fail_allocs{0};
+static std::atomic<size_t> g_ring_bytes{0};
 
 cudaError_t dev_alloc(void** p, size_t bytes) {
     int n = g_fail_allocs.load();
@@ -415,41 +416,38 @@ __global__ void k_ring_pull(uint4* __restrict__ dst, const uint4* __restrict__ s
 }
 
 int UploadRing::push(const void* src, size_t bytes, cudaStream_t st, void** dev) {
-    const size_t need = (bytes + 255) & ~(size_t)255;
-    if (need > cap || head + need > cap) {
+    size_t off = 0;
+    const size_t test_cap = g_ring_bytes.load();
+    const RingSpace was = space;
+    const RingSpace::Act act = space.place(bytes, test_cap ? test_cap : min_cap, &off);
+    if (act != RingSpace::FITS) {
         // the bytes about to be reused may still feed a copy or a kernel
-        if (last && last != st && cudaStreamSynchronize(last) != cudaSuccess) return SBG_ECUDA;
-        if (cudaStreamSynchronize(st) != cudaSuccess) return SBG_ECUDA;
-        head = 0;
-        if (need > cap) {
+        if ((last && last != st && cudaStreamSynchronize(last) != cudaSuccess) ||
+            cudaStreamSynchronize(st) != cudaSuccess) {
+            space = was;
+            return SBG_ECUDA;
+        }
+        if (act == RingSpace::GROW) {
+            const RingSpace grown = space;
             release();
-            // 32 MB: a 1024-division batch uploads about 4.5 MB of descriptors,
-            // so the ring wraps (and drains the stream) once every few calls
-            const size_t nc = std::max(need * 4, (size_t)32 << 20);
-            if (cudaHostAlloc(&h, nc, cudaHostAllocMapped) != cudaSuccess) return SBG_EALLOC;
-            if (cudaHostGetDevicePointer((void**)&hd, h, 0) != cudaSuccess) {
-                cudaFreeHost(h);
-                h = nullptr;
+            if (cudaHostAlloc(&h, grown.cap, cudaHostAllocMapped) != cudaSuccess) return SBG_EALLOC;
+            if (cudaHostGetDevicePointer((void**)&hd, h, 0) != cudaSuccess ||
+                cudaMalloc(&d, grown.cap) != cudaSuccess) {
+                release();
                 return SBG_EALLOC;
             }
-            if (cudaMalloc(&d, nc) != cudaSuccess) {
-                cudaFreeHost(h);
-                h = nullptr;
-                return SBG_EALLOC;
-            }
-            cap = nc;
+            space = grown;
         }
     }
-    std::memcpy(h + head, src, bytes);
+    std::memcpy(h + off, src, bytes);
     if (bytes) {
-        const size_t n16 = need / 16;      // the whole 256-byte-rounded block
+        const size_t n16 = RingSpace::rounded(bytes) / 16;      // the whole 256-byte-rounded block
         const unsigned blocks = (unsigned)std::min<size_t>((n16 + 255) / 256, 64);
-        k_ring_pull<<<blocks, 256, 0, st>>>((uint4*)(d + head), (const uint4*)(hd + head), n16);
+        k_ring_pull<<<blocks, 256, 0, st>>>((uint4*)(d + off), (const uint4*)(hd + off), n16);
         if (cudaGetLastError() != cudaSuccess) return SBG_ECUDA;
         ++pulls;
     }
-    *dev = d + head;
-    head += need;
+    *dev = d + off;
     last = st;
     return SBG_OK;
 }
@@ -460,7 +458,7 @@ void UploadRing::release() {
     h = nullptr;
     hd = nullptr;
     d = nullptr;
-    cap = head = 0;
+    space.clear();
 }
 
 int enqueue_products(sbg_ctx* c, const sbg_job* jobs, int64_t count, uint32_t* err) {
@@ -657,6 +655,7 @@ void sbg_ctx_destroy(sbg_ctx* c) {
     cudaFree(c->derr);
     cudaFree(c->u52buf);
     c->ring.release();
+    c->keep.release();
     for (int k = 0; k < SBG_AUX_STREAMS; ++k) {
         if (c->aux[k]) cudaStreamDestroy(c->aux[k]);
         if (c->join[k]) cudaEventDestroy(c->join[k]);
@@ -964,7 +963,7 @@ int sbg_batch_autotune(sbg_batch* b, double* ms) {
     return sbg_batch_set_engine(b, cfgs[best_i].engine, cfgs[best_i].wave ? cfgs[best_i].wave : 0);
 }
 
-int64_t sbg_ctx_launches(sbg_ctx* c) { return c ? c->launches.load() + c->ring.pulls : 0; }
+int64_t sbg_ctx_launches(sbg_ctx* c) { return c ? c->launches.load() + c->ring.pulls + c->keep.pulls : 0; }
 
 // For every size class k where a 3 * 2^k transform could replace 2^(k+2),
 // time one full product (an = bn = 3 * 2^(k-1), the largest of the class)
@@ -1155,3 +1154,5 @@ int sbg_nt_sqr(uint64_t* rp, const uint64_t* ap, ptrdiff_t an) {
 extern "C" int sbg_debug_inject(uint32_t mask) { return cuda_fail(set_inject(mask), "inject"); }
 
 extern "C" void sbg_debug_fail_allocs(int n) { g_fail_allocs.store(n < 0 ? 0 : n); }
+
+extern "C" void sbg_debug_ring_bytes(int64_t bytes) { g_ring_bytes.store(bytes < 0 ? 0 : (size_t)bytes); }

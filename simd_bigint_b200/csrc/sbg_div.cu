@@ -1141,12 +1141,14 @@ size_t div_scratch_limbs(int64_t n) { return (size_t)(14 * n + 64); }
 using namespace sbg;
 
 // Every transfer below is stream-ordered on the context stream: descriptor
-// arrays go through the context's upload ring, products through its product
-// queue; the only synchronisation is the one at the end of a call.
+// arrays go through the context's upload rings, products through its product
+// queue; the only synchronisation is the one at the end of a call.  What the
+// next launch alone reads takes the product lists' ring; what is read after
+// further product lists have been queued takes the ring that they do not use.
 template <class T>
-static int upload(sbg_ctx* c, const std::vector<T>& host, T** dev) {
+static int upload(sbg_ctx* c, const std::vector<T>& host, T** dev, bool keep = false) {
     void* d = nullptr;
-    int st = c->ring.push(host.data(), host.size() * sizeof(T), c->stream, &d);
+    int st = (keep ? c->keep : c->ring).push(host.data(), host.size() * sizeof(T), c->stream, &d);
     *dev = (T*)d;
     return st;
 }
@@ -1210,7 +1212,8 @@ static int div_core(sbg_ctx* c, std::vector<DivInst>& v, uint32_t* err, bool quo
     }
     int rc = SBG_OK;
     // Every round's descriptors are known beforehand: the base cases' and all
-    // rounds' steps go up in one piece.
+    // rounds' steps go up in one piece, which stays until the last round is
+    // queued.
     struct Round {
         std::vector<sbg_job> jt, ju;             // the two products of the divisions in it
         size_t first = 0;                        // its steps: single-CTA divisions, clustered ones
@@ -1266,7 +1269,7 @@ static int div_core(sbg_ctx* c, std::vector<DivInst>& v, uint32_t* err, bool quo
     }
     if (!steps.empty()) std::memcpy(desc.data() + soff, steps.data(), steps.size() * sizeof(RecipStep));
     uint8_t* ddesc = nullptr;
-    if ((rc = upload(c, desc, &ddesc))) return rc;
+    if ((rc = upload(c, desc, &ddesc, true))) return rc;
     if (launch_pdl(k_recip_base, true, ((int64_t)v.size() + WDIV_WARPS - 1) / WDIV_WARPS, 32 * WDIV_WARPS, 0, 1, st,
                    (const RecipBase*)ddesc, (int)v.size(), err) != cudaSuccess)
         return SBG_ECUDA;
@@ -1313,8 +1316,8 @@ static int div_core(sbg_ctx* c, std::vector<DivInst>& v, uint32_t* err, bool quo
     }
     const int fs = (int)fx.size(), fb = (int)fxb.size();
     fx.insert(fx.end(), fxb.begin(), fxb.end());
-    DivFix* dfx = nullptr;
-    if ((rc = upload(c, fx, &dfx))) return rc;
+    DivFix* dfx = nullptr;                   // every round's steps are queued: their block may go
+    if ((rc = upload(c, fx, &dfx, true))) return rc;
     if ((rc = enqueue_products(c, jp.data(), (int64_t)jp.size(), err))) return rc;
     if (!quotient) {
         if ((rc = launch_lin(c, k_recip_final<1>, k_recip_final<DIV_CL>, (const DivFix*)dfx, fs, fb, err)))

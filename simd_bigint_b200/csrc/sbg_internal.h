@@ -10,6 +10,7 @@
 
 #include "../../include/simd_bigint_b200.h"
 #include "sbg_arith.cuh"
+#include "sbg_ring.h"
 
 namespace sbg {
 
@@ -349,15 +350,19 @@ struct EventTimer : KTimer {
 
 // Stream-ordered upload of small descriptor arrays without allocation or
 // synchronisation in steady state: bytes are copied into a pinned host ring
-// and an asynchronous copy into the matching device ring is enqueued on the
-// caller's stream.  Reusing ring bytes (wrap-around) or growing the ring
-// first synchronises the streams of earlier pushes, so no copy or kernel
-// still reading the reused bytes is in flight.  One host thread at a time.
+// and a copy kernel into the matching device ring is queued on the caller's
+// stream.  Reusing ring bytes (wrap-around) or growing the ring first
+// synchronises the streams of earlier pushes, so no copy or kernel queued so
+// far still reads the reused bytes.  Kernels that are queued later are not
+// waited for: all that reads a block is queued before the next push into the
+// same ring (see RingSpace).  One host thread at a time.
 struct UploadRing {
+    explicit UploadRing(size_t least) : min_cap(least) {}
     uint8_t* h = nullptr;           // page-locked host buffer
     uint8_t* hd = nullptr;          //   its device address
     uint8_t* d = nullptr;
-    size_t cap = 0, head = 0;
+    size_t min_cap;                 // bytes of the first allocation, at least
+    RingSpace space;
     int64_t pulls = 0;              // copy kernels launched (k_ring_pull)
     cudaStream_t last = nullptr;
     int push(const void* src, size_t bytes, cudaStream_t st, void** dev);
@@ -406,10 +411,15 @@ struct sbg_ctx {
     cudaEvent_t stage_a = nullptr, stage_b = nullptr, stage_go = nullptr;
     sbg::EventTimer* timer = nullptr;    // non-null while kernel timing is on
     // queued product lists (Newton division): grow-only arena for the
-    // transforms and carry flags, descriptor ring, forked streams
+    // transforms and carry flags, descriptor ring, forked streams.  32 MB: a
+    // 1024-division batch uploads about 4.5 MB of descriptors, so the ring
+    // wraps (and drains the stream) once every few calls
     uint8_t* pw = nullptr;
     size_t pw_cap = 0;
-    sbg::UploadRing ring;
+    sbg::UploadRing ring{(size_t)32 << 20};
+    // descriptors of a division's linear steps: they are read while product
+    // lists go through `ring`, so those must not reach them (0.8 MB of the 4.5)
+    sbg::UploadRing keep{(size_t)4 << 20};
     cudaStream_t aux[SBG_AUX_STREAMS] = {};
     cudaEvent_t fork = nullptr;
     cudaEvent_t join[SBG_AUX_STREAMS] = {};
