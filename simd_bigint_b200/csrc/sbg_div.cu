@@ -1118,6 +1118,7 @@ struct DivInst {
     const uint64_t* N;      // numerator padded to 2n limbs (device), or null (recip only)
     uint64_t* Qout;         // quotient out (qlen limbs) or reciprocal out (n limbs)
     uint64_t* Rout;         // remainder out (n limbs) or null
+    uint64_t* R;            // where the last step puts the remainder: Rout, or scratch copied there
     int64_t n;
     int64_t qlen;
     // scratch (device)
@@ -1301,7 +1302,7 @@ static int div_core(sbg_ctx* c, std::vector<DivInst>& v, uint32_t* err, bool quo
             }
         }
         F.Q = d.Q;
-        F.R = quotient ? d.Rout : d.Qout;
+        F.R = quotient ? d.R : d.Qout;
         F.Rw = d.Rw;
         F.n = d.n;
         uint64_t* X = d.X[0];
@@ -1331,9 +1332,11 @@ static int div_core(sbg_ctx* c, std::vector<DivInst>& v, uint32_t* err, bool quo
         if ((rc = enqueue_products(c, jq.data(), (int64_t)jq.size(), err))) return rc;
         if ((rc = launch_lin(c, k_div_fix<1>, k_div_fix<DIV_CL>, (const DivFix*)dfx, fs, fb, err))) return rc;
         std::vector<CopyDesc> cq;
-        cq.reserve(v.size());
-        for (auto& d : v)
+        cq.reserve(2 * v.size());
+        for (auto& d : v) {
             if (d.Q != d.Qout) cq.push_back(CopyDesc{d.Q, d.Qout, d.qlen, d.qlen});
+            if (d.R != d.Rout) cq.push_back(CopyDesc{d.R, d.Rout, d.n, d.n});
+        }
         if ((rc = copy_batch(c, cq))) return rc;
     }
     return SBG_OK;
@@ -1483,6 +1486,9 @@ static int divrem_enqueue(sbg_ctx* c, const sbg_div_job* jobs, int64_t count, bo
     // divisions of mixed sizes, 4942 -> 4818 us without the copies.
     // Shorter numerators need the zero limbs above them, shorter quotients room
     // for a top limb that is zero only after the correction.
+    // Likewise the last step writes the remainder while it still reads the
+    // divisor: unless all outputs are apart, it goes to scratch and from there,
+    // once no kernel reads an operand any more, to its place.
     const bool apart = outputs_apart(jobs, count);
     for (int64_t i = 0; i < count; ++i) {
         const sbg_div_job& j = jobs[i];
@@ -1500,6 +1506,7 @@ static int divrem_enqueue(sbg_ctx* c, const sbg_div_job* jobs, int64_t count, bo
             d.N = j.np;
             carve(d, p);
             d.Q = j.qp;
+            d.R = j.rp;
             continue;
         }
         // numerator zero-padded to 2n limbs (one batched copy below)
@@ -1508,6 +1515,7 @@ static int divrem_enqueue(sbg_ctx* c, const sbg_div_job* jobs, int64_t count, bo
         cn.back() = CopyDesc{j.np, Np, j.nn, 2 * j.dn};
         d.N = Np;
         carve(d, p);
+        d.R = apart ? j.rp : d.T;           // T is done with by then
     }
     rc = copy_batch(c, cn);
     if (!rc) rc = div_core(c, v, c->derr, true);
