@@ -1092,8 +1092,8 @@ __global__ void __launch_bounds__(DIV_T) k_recip_final(const DivFix* df, uint32_
     // Q holds X (n+1 limbs); V = X (+1) low n limbs
     uint64_t* Q = F.Q;
     const uint64_t q0 = Q[0];
+    grp.sync();                             // limb 0 and D, over which the result may go, are read
     if (c >= 0 && q0 == ~0ull) {
-        grp.sync();                         // every CTA has read limb 0
         block_step1(grp, Q, n + 1, true);
         grp.sync();
         if (threadIdx.x == 0 && Q[n] != 1) atomicOr(err, 64u);

@@ -66,3 +66,20 @@ def test_results_over_the_divisor(ctx, n, layout):
     for i in range(len(divs)):
         wq, wr = divmod(_int(nums[i]), _int(divs[i]))
         assert _host(q[i]) == wq and _host(r[i]) == wr, i
+
+
+@pytest.mark.parametrize("n", [100, 128, 700, 6200, 9000, 40000])
+def test_reciprocals_in_place(ctx, n):
+    import torch
+    B = 1 << 64
+    rng = np.random.default_rng(n + 3)
+    r = _int(rng.integers(0, 2**64, n, dtype=np.uint64))
+    # divisors whose reciprocal ends in zeros or ones, and a random one
+    for d in (B**n // 2, B**n // 2 + 1, B**n - 1, r | B**n // 2, (2 * B**n) // 3 | B**n // 2):
+        for shift in (0, 17):
+            buf = torch.zeros(n + 17, dtype=torch.int64, device="cuda")
+            buf[:n] = _dev(_limbs(d, n))
+            v = buf[shift:shift + n]
+            torch.cuda.synchronize()
+            ctx.recip(v, buf[:n])
+            assert _host(v) == ((1 << (128 * n)) - 1) // d - (1 << (64 * n)), shift
