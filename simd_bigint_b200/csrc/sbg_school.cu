@@ -47,8 +47,10 @@ __global__ void __launch_bounds__(SCHOOL_T) k_school(const uint64_t* __restrict_
     const int step = wid % SCHOOL_STEPS, part = wid / SCHOOL_STEPS;
     const int n = an + bn;
     pdl_enter();
-    for (int i = tid; i < 3 * MAX; i += SCHOOL_T) sb[i] = i >= MAX && i < MAX + bn ? __ldg(&b[i - MAX]) : 0;
-    if (tid < an) sa[tid] = __ldg(&a[tid]);
+    // the kernel before may have written the operands while this one was
+    // already resident: not through the read-only path
+    for (int i = tid; i < 3 * MAX; i += SCHOOL_T) sb[i] = i >= MAX && i < MAX + bn ? __ldcg(&b[i - MAX]) : 0;
+    if (tid < an) sa[tid] = __ldcg(&a[tid]);
     if (tid < 3) {
         c_lo[tid] = c_mid[tid] = 0;
         c_hi[tid] = 0;
