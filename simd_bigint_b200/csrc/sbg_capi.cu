@@ -131,11 +131,28 @@ static int ensure_ws(sbg_ctx* c, size_t words, size_t flag_words) {
     return SBG_OK;
 }
 
+// the product lists' grow-only arena, `words` u32 words and a quarter more
+static int ensure_arena(sbg_ctx* c, size_t words) {
+    const size_t bytes = words * sizeof(uint32_t);
+    if (bytes <= c->pw_cap) return SBG_OK;
+    // earlier lists on this stream may still use the arena
+    CK(cudaStreamSynchronize(c->stream));
+    cudaFree(c->pw);
+    c->pw = nullptr;
+    c->pw_cap = 0;
+    const size_t nb = bytes + bytes / 4;
+    CK(cudaMalloc(&c->pw, nb));
+    c->pw_cap = nb;
+    return SBG_OK;
+}
+
 // One windowed convolution: the limbs [off, off + nout) of
 // sum_{cmin <= j <= cmax} c_j 2^(64 j) where c = a * b (cyclic length 2^lgL).
+// In the product lists' arena if `arena`, which longer lists have mostly grown
+// already, else in the workspace of the context's own products.
 static int run_conv(sbg_ctx* c, uint64_t* rp, const uint64_t* ap, int64_t an, const uint64_t* bp,
                     int64_t bn, int sq, int lgL, int64_t cmin, int64_t cmax, int64_t off,
-                    int64_t nout, cudaEvent_t b_ready = nullptr, uint32_t* err = nullptr) {
+                    int64_t nout, cudaEvent_t b_ready = nullptr, uint32_t* err = nullptr, bool arena = false) {
     if (!err) err = c->err;
     if (lgL > SBG_NCODES || code_len(lgL) > ((int64_t)1 << SBG_MAX_LG)) return SBG_EBAND;
     int st = ensure_plan(c, lgL);
@@ -157,13 +174,15 @@ static int run_conv(sbg_ctx* c, uint64_t* rp, const uint64_t* ap, int64_t an, co
         c->launches += 1;
         return SBG_OK;
     }
-    st = ensure_ws(c, ws_words(lgL, sq), carry_flag_words(nout));
+    const size_t words = ws_words(lgL, sq), flag_words = carry_flag_words(nout);
+    st = arena ? ensure_arena(c, words + flag_words) : ensure_ws(c, words, flag_words);
     if (st) return st;
+    uint32_t* ws = arena ? (uint32_t*)c->pw : c->ws;
+    uint32_t* flags = arena ? ws + words : c->flags;
     const LenPlan* lp = &c->plans[lgL];
-    CK(launch_conv(ap, an, bp, bn, sq, lgL, lp, c->tw_f, c->tw_i, c->ws, c->flags,
-                   (int64_t)carry_flag_words(nout), c->stream, c->timer, b_ready));
-    CK(launch_crt_carry(c->ws, lgL, lp, cmin, cmax, off, rp, nout, c->flags, err, c->stream,
-                        c->timer));
+    CK(launch_conv(ap, an, bp, bn, sq, lgL, lp, c->tw_f, c->tw_i, ws, flags, (int64_t)flag_words, c->stream, c->timer,
+                   b_ready));
+    CK(launch_crt_carry(ws, lgL, lp, cmin, cmax, off, rp, nout, flags, err, c->stream, c->timer));
     // the split forward columns (b_ready on the four-step path) are two launches
     c->launches += class_launches(lgL) + ((b_ready && !sq && lgL > SBG_SMALL_MAX_LG && lp->m3 < 0) ? 1 : 0);
     return SBG_OK;
@@ -475,7 +494,7 @@ int enqueue_products(sbg_ctx* c, const sbg_job* jobs, int64_t count, uint32_t* e
         const uint64_t* bp = sq ? j.ap : j.bp;
         const int64_t bn = sq ? j.an : j.bn;
         if (lgL == SBG_CODE_SCHOOL) return run_school(c, j.rp, j.ap, j.an, bp, bn);
-        return run_conv(c, j.rp, j.ap, j.an, bp, bn, sq, lgL, cmin, cmax, off, nout, nullptr, err);
+        return run_conv(c, j.rp, j.ap, j.an, bp, bn, sq, lgL, cmin, cmax, off, nout, nullptr, err, true);
     }
     std::vector<JobDesc> by_lg[SBG_NCODES + 1];
     int64_t max_nout[SBG_NCODES + 1] = {};
@@ -503,17 +522,8 @@ int enqueue_products(sbg_ctx* c, const sbg_job* jobs, int64_t count, uint32_t* e
         for (auto& d : by_lg[l]) ws_total += ws_words(l, d.sq);
         flag_total += by_lg[l].size() * ((size_t)crt_blocks(max_nout[l]) + 1 + 3) / 4 * 4;
     }
-    const size_t bytes = (ws_total + flag_total) * 4;
-    if (bytes > c->pw_cap) {
-        // earlier lists on this stream may still use the arena
-        CK(cudaStreamSynchronize(c->stream));
-        cudaFree(c->pw);
-        c->pw = nullptr;
-        c->pw_cap = 0;
-        const size_t nb = bytes + bytes / 4;
-        CK(cudaMalloc(&c->pw, nb));
-        c->pw_cap = nb;
-    }
+    int st = ensure_arena(c, ws_total + flag_total);
+    if (st) return st;
     if (!c->fork) {
         for (int k = 0; k < SBG_AUX_STREAMS; ++k) {
             CK(cudaStreamCreateWithPriority(&c->aux[k], cudaStreamNonBlocking, c->stream_priority));
@@ -549,7 +559,7 @@ int enqueue_products(sbg_ctx* c, const sbg_job* jobs, int64_t count, uint32_t* e
         }
     }
     void* dd = nullptr;
-    int st = c->ring.push(all.data(), all.size() * sizeof(JobDesc), c->stream, &dd);
+    st = c->ring.push(all.data(), all.size() * sizeof(JobDesc), c->stream, &dd);
     if (st) return st;
     // a list of one class stays on the context's stream
     const int nst = cls.size() == 1 ? 0 : std::min<int>(SBG_AUX_STREAMS, (int)cls.size());
