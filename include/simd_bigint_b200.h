@@ -77,8 +77,9 @@ int sbg_ctx_set_timing(sbg_ctx *ctx, int on);
 /* Number of kernel launches this context has queued so far (diagnostics). */
 int64_t sbg_ctx_launches(sbg_ctx *ctx);
 /* Transform lengths.  A product of N coefficients runs at L = 2^a >= N or,
- * for 2^(k+1) < N <= 3 * 2^k, at L = 3 * 2^k: always for 12 <= k <= 15, and
- * for 16 <= k <= 23 when bit k of the context's mask is set.
+ * for 2^(k+1) < N <= 3 * 2^k, at L = 3 * 2^k: for 16 <= k <= 23 when bit k of
+ * the context's mask is set, for 12 <= k <= 15 unless the mask is 0 (powers of
+ * two alone, which one persistent kernel runs for a whole batch).
  * sbg_ctx_autotune times one product of each of those eight size classes at
  * both lengths on this device (about a second; allocates 400 MB temporarily)
  * and sets the mask to the faster; times (optional, 16 doubles) receives

@@ -45,15 +45,15 @@ int lg_ceil(int64_t n) {
 }
 
 // Transform length (code) for a convolution whose wanted coefficients need
-// L >= need: 2^a >= need, or 3 * 2^b >= need when that is shorter and b is
-// 12 .. 15, or bit b of `mask3` allows it (the context's choice per size
-// class, sbg_ctx_autotune).
+// L >= need: 2^a >= need, or 3 * 2^b >= need when that is shorter and bit b
+// of `mask3` allows it (the context's choice per size class,
+// sbg_ctx_autotune); b = 12 .. 15, which have no bit, unless the mask is 0.
 int conv_lg(int64_t need, uint32_t mask3) {
     int l = lg_ceil(need);
     if (l < 4) l = 4;
     int k = lg_ceil((need + 2) / 3);
     if (k >= SBG_THREE_SHORT_LG && k <= SBG_MAX_LG - 2 && ((int64_t)3 << k) < ((int64_t)1 << l) &&
-        (k < SBG_THREE_MIN_LG || ((mask3 >> k) & 1u)))
+        (k < SBG_THREE_MIN_LG ? mask3 != 0 : ((mask3 >> k) & 1u) != 0))
         return SBG_CODE3 + k;
     return l;
 }

@@ -72,8 +72,9 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), bool pdl, int64_t blocks, 
 #define SBG_CODE3 32
 #define SBG_NCODES (SBG_CODE3 + SBG_MAX_LG)
 #define SBG_THREE_MIN_LG 16
-// k = 12 .. 15 are always used: their columns have at most 24 rows, so the
-// radix-3 level needs no exchange and the quarter of the points saved is saved
+// k = 12 .. 15 are used unless the mask is 0: their columns have at most 24
+// rows, so the radix-3 level needs no exchange and the quarter of the points
+// saved is saved
 #define SBG_THREE_SHORT_LG 12
 // k = 16..19 and 21..23: where 3 * 2^k measured faster than 2^(k+2) on B200
 // (at k = 20 the columns of 768 rows need the cross-CTA radix-3 exchange,
