@@ -47,10 +47,23 @@ namespace cg = cooperative_groups;
 // rounds, where few divisions remain -- spread over DIV_CL SMs.
 #define DIV_CL 8
 #define DIV_CL_MIN_N 32768
-// Where at most DIV_CL_FEW divisions are in a step, clusters of them fit on
-// the device side by side and shorter ones are spread as well.
+// Where at most DIV_CL_FEW divisions are in a step, clusters of them fit on the
+// device side by side and shorter ones are spread as well: from 6144 limbs, and
+// from 1024 for each division, since more of them fill more of the device as
+// they are.  us a batch of divisions of n limbs with the line at 32768 / at 6144
+// whatever their number / here: 4 x 6200 439 / 455 / 453, 4 x 9000 498 / 496 /
+// 488, 4 x 30000 749 / 683 / 694, 8 x 18000 716 / 694 / 685, 12 x 14000 662 /
+// 643 / 637, 16 x 6200 538 / 570 / 535, 16 x 7000 555 / 584 / 548, 16 x 9000
+// 648 / 656 / 637; a reciprocal of 100000 limbs 544 / 510 / 508.  A line at 1024
+// costs (16 x 4500: 510 -> 556), and more than 16 divisions gain nothing (24 x
+// 20000 959 / 960, 32 x 20000 1073 / 1120, 64 x 9000 1005 / 1150).
 #define DIV_CL_FEW 16
 #define DIV_CL_FEW_MIN_N 6144
+#define DIV_CL_FEW_PER 1024
+// the least n whose steps run on a cluster where `live` divisions are in a step
+static int64_t cluster_min(int64_t live) {
+    return live <= DIV_CL_FEW ? std::max<int64_t>(DIV_CL_FEW_MIN_N, DIV_CL_FEW_PER * live) : DIV_CL_MIN_N;
+}
 
 // The CTA group of one division: its rank, a barrier over all of its
 // threads (release / acquire: global and shared memory written before it
@@ -1228,7 +1241,7 @@ static int div_core(sbg_ctx* c, std::vector<DivInst>& v, uint32_t* err, bool quo
         R.first = steps.size();
         int live = 0;
         for (auto& d : v) live += (int)d.sz.size() - 1 >= r;
-        const int64_t cl_min = live <= DIV_CL_FEW ? DIV_CL_FEW_MIN_N : DIV_CL_MIN_N;
+        const int64_t cl_min = cluster_min(live);
         for (auto& d : v) {
             const int depth = (int)d.sz.size() - 1;
             if (depth < r) continue;
@@ -1287,7 +1300,7 @@ static int div_core(sbg_ctx* c, std::vector<DivInst>& v, uint32_t* err, bool quo
     if (rc) return rc;
     // final stage: exact reciprocal, or quotient and remainder
     std::vector<DivFix> fx, fxb;             // single-CTA divisions, clustered ones
-    const int64_t cl_min = v.size() <= DIV_CL_FEW ? DIV_CL_FEW_MIN_N : DIV_CL_MIN_N;
+    const int64_t cl_min = cluster_min((int64_t)v.size());
     std::vector<sbg_job> jp;
     for (auto& d : v) {
         DivFix F{};
