@@ -1904,6 +1904,12 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
     const int lgN1 = lp->lgN1;   // rows: 2^lgN1 (or 3 * 2^m3), columns: 2^12
     const int m3 = lp->m3;
     const int nops = sq ? 1 : 2;
+    // Kernels that are let in early are placed on the SMs that empty first.  With
+    // one or two column CTAs per SM that leaves some SMs with several and others
+    // with none, and the kernel lasts as long as the fullest: from 3 * 2^16 to
+    // 3 * 2^17 points the forward columns (80 to 320 CTAs) start whole, at
+    // 3 * 2^17 the inverse ones (160) too.
+    const bool pdl_f = pdl && !(L > ((size_t)1 << 17) && L < ((size_t)1 << 19)), pdl_i = pdl && m3 != 5;
     cudaError_t e = cudaSuccess;
     if (m3 >= 0) {
         const Radix3Arg r3f = radix3_arg(lp, false), r3i = radix3_arg(lp, true);
@@ -1911,7 +1917,7 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
         switch (m3) {
 #define SBG_LAUNCH_F3S(n)                                                                          \
     case n:                                                                                        \
-        e = launch_colx(k_col3s_fwd<n>, pdl, (int64_t)nops * col3s_ntiles(n) * SBG_NP, col3s_smem_bytes(n), 1, \
+        e = launch_colx(k_col3s_fwd<n>, pdl_f, (int64_t)nops * col3s_ntiles(n) * SBG_NP, col3s_smem_bytes(n), 1, \
                         st, a, an, b, bn, tw_f, r3f, YA, YB);                                       \
         break;
             SBG_COL3S_CASES(SBG_LAUNCH_F3S)
@@ -1942,7 +1948,7 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
         switch (m3) {
 #define SBG_LAUNCH_I3S(n)                                                                          \
     case n:                                                                                        \
-        e = launch_colx(k_col3s_inv<n>, pdl, (int64_t)col3s_ntiles(n) * SBG_NP, col3s_smem_bytes(n), 1, st, YA, \
+        e = launch_colx(k_col3s_inv<n>, pdl_i, (int64_t)col3s_ntiles(n) * SBG_NP, col3s_smem_bytes(n), 1, st, YA, \
                         tw_i, r3i);                                                                 \
         break;
             SBG_COL3S_CASES(SBG_LAUNCH_I3S)
@@ -1986,7 +1992,7 @@ cudaError_t launch_conv(const uint64_t* a, int64_t an, const uint64_t* b, int64_
             if (e == cudaSuccess)                                                                \
                 e = launch_col(k_col_fwd<n>, pdl, n, col_blocks, st, b, bn, b, bn, tw_f, YB, YB, 1);    \
         } else {                                                                                 \
-            e = launch_col(k_col_fwd<n>, pdl, n, nops * col_blocks, st, a, an, b, bn, tw_f, YA, YB, nops); \
+            e = launch_col(k_col_fwd<n>, pdl_f, n, nops * col_blocks, st, a, an, b, bn, tw_f, YA, YB, nops); \
         }                                                                                        \
         break;
         SBG_COL_CASES(SBG_LAUNCH_F)
@@ -2060,7 +2066,8 @@ cudaError_t launch_batch_class(const JobDesc* djobs, int njobs, int lgL, const L
         sc.ws[q] = lp->scale[q].ws;
     }
     cudaError_t e = cudaSuccess;
-    const bool pdl = alone && (int64_t)njobs * code_len(lgL) <= SBG_PDL_POINTS;
+    const int64_t rows = SBG_NP * (code_len(lgL) >> ROW_LG) * njobs;    // 0: one-CTA and cluster products
+    const bool pdl = alone && rows <= ROWL_MAX && (int64_t)njobs * code_len(lgL) <= SBG_PDL_POINTS;
     KT_BEGIN(kt, KID_BATCH, st);
     if (lgL >= SBG_FUSED_MIN_LG && lgL <= SBG_SMALL_MAX_LG) {
         switch (lgL) {
