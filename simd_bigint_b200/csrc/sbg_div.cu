@@ -974,7 +974,7 @@ __global__ void __launch_bounds__(DIV_T) k_div_fix(const DivFix* df, uint32_t* e
     uint64_t f0 = 0, f1 = 0, f2 = 0, f3 = 0;
     if (F.L > 0 && n >= 4) {
         const int64_t L = F.L;
-        const __int128 top = (__int128)N[L - 1] + (2 * L - 1 < 2 * n ? N[2 * L - 1] : 0) - P[L - 1];
+        const __int128 top = (__int128)N[L - 1] - P[L - 1];        // N_hi has no limb L-1: L >= n + 3
         const __int128 d = (top + ((__int128)1 << 63)) >> 64;
         const __int128 off = top - (d << 64);
         settled = off >= -4 && off <= 4 && d >= -2 && d <= 2;
