@@ -24,11 +24,11 @@ def test_workspace_is_not_grown():
     L = sbg.lib()
     rng = np.random.default_rng(11)
     try:
-        # the tables of every length below, without a workspace
+        # the tables of every length below, without a workspace (a batch each:
+        # in one, short lengths join longer ones)
         x = torch.zeros(1 << 17, dtype=torch.int64, device="cuda")
-        jobs = [(sbg.JOB_MUL, x.data_ptr(), x.data_ptr(), x.data_ptr(), ln, 1)
-                for ln in [1 << k for k in range(7, 17)] + [3 << k for k in range(12, 15)]]
-        sbg.Batch(ctx, jobs).close()
+        for ln in [1 << k for k in range(7, 17)] + [3 << k for k in range(12, 15)]:
+            sbg.Batch(ctx, [(sbg.JOB_MUL, x.data_ptr(), x.data_ptr(), x.data_ptr(), ln, 1)]).close()
         d = rand_limbs(n, rng)
         d[-1] |= np.uint64(1 << 63)
         a, b = rand_limbs(9000, rng), rand_limbs(8000, rng)
