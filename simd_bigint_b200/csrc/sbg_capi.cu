@@ -188,7 +188,7 @@ static int run_conv(sbg_ctx* c, uint64_t* rp, const uint64_t* ap, int64_t an, co
     return SBG_OK;
 }
 
-// A plain product of at most SBG_SCHOOL_MAX limbs: one schoolbook warp.
+// A plain product of at most SBG_SCHOOL_MAX limbs: schoolbook on one CTA.
 static int run_school(sbg_ctx* c, uint64_t* rp, const uint64_t* ap, int64_t an, const uint64_t* bp,
                       int64_t bn) {
     KT_BEGIN(c->timer, KID_SMALL, c->stream);

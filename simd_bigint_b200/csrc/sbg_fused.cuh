@@ -294,9 +294,10 @@ __global__ void __launch_bounds__(fu_threads(LG), 1024 / fu_threads(LG))
 // Columns of 2 to 16 rows of a single product: a thread per column and prime,
 // 128 threads a CTA.  The general column kernels' tiles hold 2^13 points, which
 // at two rows leaves ten CTAs for both operands; here there are 320 whatever
-// the length.  2 rows (8192 points): forward 10.1 -> 3.9 us, inverse 10.8 -> 3.6;
-// 8 rows: 5.5 -> 4.1 and 5.5 -> 3.8.  Batches keep the tiles: their jobs fill
-// the device, and a CTA per 128 columns would cost them more launches than work.
+// the length.  Launches as the profiler times them: 2 rows (8192 points) forward
+// 10.6 -> 3.2 us, inverse 11.1 -> 2.9; 8 rows 6.0 -> 3.8 and 5.8 -> 3.6; 16 rows
+// 5.9 -> 4.6 and 4.8 -> 5.0.  Batches keep the tiles: their jobs fill the device,
+// and a CTA per 128 columns would cost them more launches than work.
 // ------------------------------------------------------------------------
 #define COLN_T 128
 #define COLN_MAX_LG 4

@@ -35,10 +35,13 @@ __device__ __forceinline__ void pdl_enter() {
 // beside the chain: single products of up to SBG_PDL_POINTS transform points
 // (16384 x 16384 limbs: 29.5 -> 20.3 us a call with it and without the flags'
 // memset, 333333 x 77777: 65.5 -> 59.6; at 2^24 x 2^20, where the waiting CTAs
-// only take room, 2605 -> 2674) and product lists of one length class (a
-// reciprocal of 100000 limbs: 1348 -> 1217 us).  In a batch of several
-// classes the waiting CTAs of one stream keep other streams' kernels out (1024
-// products: 1352 -> 1363 us), so there it is off.
+// only take room, 2605 -> 2674; launch_conv names the kernels left out), the
+// Newton steps (a reciprocal of 100000 limbs: 1348 -> 1217 us) and batches of
+// one length class of at most one row per SM.  With more rows the column CTAs
+// let in early crowd on some SMs (a graph of 2 products of 60000 limbs: 34.9
+// us without, 41.0 with), and in a batch of several classes the waiting CTAs of
+// one stream keep other streams' kernels out (1024 products: 1352 -> 1363 us),
+// so there it is off.
 #define SBG_PDL_POINTS ((int64_t)1 << 20)
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kern)(KArgs...), bool pdl, int64_t blocks, int threads, size_t smem, int cluster,
@@ -81,7 +84,7 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), bool pdl, int64_t blocks, 
 // which costs more than the quarter of the points it saves)
 #define SBG_LEN3_DEFAULT 0x00EF0000u
 // Plain products of at most SBG_SCHOOL_MAX limbs (an + bn) run as one
-// schoolbook warp each (sbg_school.cu); in the batch engine they form the
+// schoolbook warp each, or a CTA where there is one alone (sbg_school.cu); in the batch engine they form the
 // length class SBG_CODE_SCHOOL (no transform, no workspace).
 #define SBG_SCHOOL_MAX 128
 #define SBG_CODE_SCHOOL 1
@@ -377,7 +380,9 @@ struct UploadRing {
 #define SBG_JOB_CYCLIC 0x43
 
 #define SBG_AUX_STREAMS 4
-// transforms up to 2^12 points run in one CTA per prime (k_small)
+// transforms up to 2^12 points run without the four-step split: a five-CTA cluster
+// for the whole product from 2^8 points on (k_fused), below that and for the
+// allocation-free multiply one CTA per prime (k_small)
 #define SBG_SMALL_MAX_LG 12
 
 // kernel launches of one product (or one length class of a batch): the

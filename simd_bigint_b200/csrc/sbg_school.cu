@@ -1,5 +1,6 @@
 // sbg_school.cu -- the small-size front end: schoolbook products of at most
-// SBG_SCHOOL_MAX output limbs, one warp per product.
+// SBG_SCHOOL_MAX output limbs, one warp per product in batches, one CTA for a
+// product alone.
 //
 // Below a few dozen limbs a five-prime transform is all overhead (five CTAs,
 // three transforms and a CRT launch for a handful of limbs).  The reference
@@ -28,8 +29,9 @@ namespace sbg {
 // (part, step) accumulates every SCHOOL_PARTS-th term of the 32 columns of its
 // step, the parts' sums meet in shared memory and one warp per step resolves
 // its limbs.  b sits between zeros, so a lane's terms need no range test.
-// 60 x 40 limbs: 12.3 -> 4.1 us of device time a call, back to back, against the one-warp form,
-// which batches keep (there the products fill the device).
+// 60 x 40 limbs against the one-warp form, which batches keep (there the products
+// fill the device): 12.3 -> 4.1 us a call back to back, the host's pace; 6.0 ->
+// 2.0 us in a captured chain of them.
 #define SCHOOL_PARTS 4
 #define SCHOOL_STEPS (SBG_SCHOOL_MAX / 32)
 #define SCHOOL_T (32 * SCHOOL_PARTS * SCHOOL_STEPS)

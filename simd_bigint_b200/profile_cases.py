@@ -6,11 +6,10 @@ command, for capturing them under a profiler:
 Cases (operands seeded, resident on cuda:0, each call repeated `repeats`
 times, 3 by default, so a capture can skip the first launch):
 
-    small     one 1500 x 1500-limb product (one launch, k_fused;
-              the short-product carry scan k_crt_carry_s)
-    mid       one 16384 x 16384-limb product (four-step kernels at 2^15
-              points, k_crt_carry_s)
-    school    one 40 x 60-limb product (schoolbook warp, k_school)
+    small     one 1500 x 1500-limb product (one launch, k_fused)
+    mid       one 16384 x 16384-limb product (k_coln, k_rowl at 2^15 points,
+              then k_crt_carry_s)
+    school    one 40 x 60-limb product (schoolbook on one CTA, k_school)
     batch     a 512-product mixed batch on the per-class engine (k_*_b)
     persist   the same batch on the persistent queue kernel (k_persist)
     divwarp   256 divisions of 200 by 100 limbs (warp block division)
